@@ -280,6 +280,19 @@ cudaError_t enqueue_ssp2_part(mth_handle* h, double dt, int part);
 // whose ghosts the boundary conditions filled, U += dt/2 S, finalise.
 cudaError_t rksplit2_half_source(mth_handle* h, double dt) {
   cudaError_t e;
+  if (h->cfg.model == MTH_HYBRID && !h->g.functional_sigma) {
+    // one pass over the cells; of the ghosts only the REGIME term's stencil
+    // reads any, and of prims alone
+    const RegimeWork* w = h->cfg.regime ? &h->regime : nullptr;
+    if (w && (e = launch_apply_bcs(h->g, h->prims, h->NP, h->st))) return e;
+    if ((e = timed(h, "source", 2.0 * h->NC, [&] {
+           return launch_hybrid_source_add(h->g, h->cfg.weno_order, h->cons, h->prims, h->aux, w,
+                                           h->hext, h->cfg.precision == MTH_MIXED, 0.5 * dt,
+                                           h->st);
+         })))
+      return e;
+    return c2p(h, h->cons, h->prims, h->aux, h->prims, h->aux);
+  }
   if ((e = launch_apply_bcs(h->g, h->cons, h->NC, h->st)) ||
       (e = launch_apply_bcs(h->g, h->prims, h->NP, h->st)) ||
       (e = launch_apply_bcs(h->g, h->aux, h->NA, h->st)))

@@ -49,73 +49,105 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// Hybrid::finalise (hybrid.cc:474-503) of one cell: E blended towards -v x B.
+__device__ __forceinline__ void finalise_e(double iW, const double* p, const double* E,
+                                           double* out) {
+  const double iE[3] = {-(p[2] * p[7] - p[3] * p[6]), -(p[3] * p[5] - p[1] * p[7]),
+                        -(p[1] * p[6] - p[2] * p[5])};
+  for (int v = 0; v < 3; ++v) {
+    double e = E[v];
+    e *= (1 - iW);
+    e += iW * iE[v];
+    out[v] = e;
+  }
+}
+
 // Hybrid::getPrimitiveVars (hybrid.cc:354-436) on interior cells: B and E
 // taken from cons, then the resistive recovery where the conductivity is
 // below sigmaCrossOver, else SRMHD's single-cell recovery (hybrd1, tol 1.4e-8,
-// srmhd.cc:297-377) of the ideal variables and its conversion back.
-__global__ void __launch_bounds__(kThreads)
-    k_hybrid_c2p(Grid g, const double* __restrict__ cons, const double* prims_guess,
-                 const double* aux_guess, double* prims, double* aux, C2PWork w) {
+// srmhd.cc:297-377) of the ideal variables and its conversion back; then
+// Hybrid::finalise of the cell, which reads only its own values.
+// Bound by the solver's FP64 latency.  The statistics take one atomic per
+// warp: one per cell on the same two words had taken longer than the solves
+// (with finalise folded in and the source step in one pass, the 512 x 500
+// RKSplit2 + REGIME step went from 1.64 to 0.96 ms).  128 registers (4 CTAs
+// per SM) 0.960 ms, 80 0.967, 64 0.970: nothing gained by more warps.
+__global__ void __launch_bounds__(kThreads, 4)
+    k_hybrid_c2p(Grid g, double* cons, const double* prims_guess, const double* aux_guess,
+                 double* prims, double* aux, C2PWork w) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= n_interior(g)) return;
-  int i, j, k;
-  interior_ijk(g, t, i, j, k);
-  const long long N = g.Ntot, cell = cell_id(g, i, j, k);
-  double c[14], p[11], a[17];
-  for (int v = 0; v < 14; ++v) c[v] = cons[v * N + cell];
-  for (int v = 5; v < 11; ++v) p[v] = c[v];
-  bool ok;
+  const bool active = t < n_interior(g);
   long long evals = 0;
-  // Each branch reads only the guesses its recovery uses: the secant on Z
-  // its aux[10] (and it writes all of prims and aux), SRMHD's hybrd1 the
-  // velocity, density and enthalpy of the ideal variables, which
-  // Hybrid::setIdealCPAs copies from the resistive prims[0..3] and aux[0].
-  if (sigma_of(g, c[0]) < g.sigma_cross) {
-    a[10] = aux_guess[10 * N + cell];
-    int ev = 0;
-    ok = srrmhd::c2p_cell(c, g.gamma, sigma_of(g, c[0]), p, a, ev);
-    evals = ev;
-  } else {
-    double ic[9], ip[8], ia[13];
-    for (int v = 0; v < 8; ++v) ic[v] = c[v];
-    ic[8] = c[12];
-    for (int v = 0; v < 4; ++v) ip[v] = prims_guess[v * N + cell];
-    ia[0] = aux_guess[cell];
-    srmhd::Residual R = srmhd::residual_args(ic, g.gamma);
-    double x[2], fv[2];
-    srmhd::guess_from_prims(ip, ia[0], x);
-    const HybrdResult res = Hybrd<2>::solve(R, x, fv, 1.4e-8);
-    evals = res.nfev;
-    ok = res.info == 1;
+  if (active) {
+    int i, j, k;
+    interior_ijk(g, t, i, j, k);
+    const long long N = g.Ntot, cell = cell_id(g, i, j, k);
+    double c[14], p[11], a[17];
+    for (int v = 0; v < 14; ++v) c[v] = cons[v * N + cell];
+    for (int v = 5; v < 11; ++v) p[v] = c[v];
+    bool ok;
+    // Each branch reads only the guesses its recovery uses: the secant on Z
+    // its aux[10] (and it writes all of prims and aux), SRMHD's hybrd1 the
+    // velocity, density and enthalpy of the ideal variables, which
+    // Hybrid::setIdealCPAs copies from the resistive prims[0..3] and aux[0].
+    if (sigma_of(g, c[0]) < g.sigma_cross) {
+      a[10] = aux_guess[10 * N + cell];
+      int ev = 0;
+      ok = srrmhd::c2p_cell(c, g.gamma, sigma_of(g, c[0]), p, a, ev);
+      evals = ev;
+    } else {
+      double ic[9], ip[8], ia[13];
+      for (int v = 0; v < 8; ++v) ic[v] = c[v];
+      ic[8] = c[12];
+      for (int v = 0; v < 4; ++v) ip[v] = prims_guess[v * N + cell];
+      ia[0] = aux_guess[cell];
+      srmhd::Residual R = srmhd::residual_args(ic, g.gamma);
+      double x[2], fv[2];
+      srmhd::guess_from_prims(ip, ia[0], x);
+      const HybrdResult res = Hybrd<2>::solve(R, x, fv, 1.4e-8);
+      evals = res.nfev;
+      ok = res.info == 1;
+      if (ok) {
+        srmhd::from_solution(ic, x, g.gamma, R.BS, R.Bsq, R.Ssq, ip, ia);
+        for (int v = 0; v < 8; ++v) p[v] = ip[v];
+        a[0] = ia[0]; a[1] = ia[1]; a[2] = ia[2]; a[3] = ia[3];
+        a[4] = 0; a[5] = 0; a[6] = 0; a[7] = ia[11];
+        a[8] = c[8] * c[8] + c[9] * c[9] + c[10] * c[10];
+        a[9] = ia[9];
+        a[10] = p[0] * a[0] * a[1] * a[1];
+        a[11] = p[1] * c[8] + p[2] * c[9] + p[3] * c[10];
+        a[12] = a[10] * p[1];
+        a[13] = a[10] * p[2];
+        a[14] = a[10] * p[3];
+        a[15] = a[12] * a[12] + a[13] * a[13] + a[14] * a[14];
+        a[16] = a[10] - p[4] - c[0];
+      }
+    }
     if (ok) {
-      srmhd::from_solution(ic, x, g.gamma, R.BS, R.Bsq, R.Ssq, ip, ia);
-      for (int v = 0; v < 8; ++v) p[v] = ip[v];
-      a[0] = ia[0]; a[1] = ia[1]; a[2] = ia[2]; a[3] = ia[3];
-      a[4] = 0; a[5] = 0; a[6] = 0; a[7] = ia[11];
-      a[8] = c[8] * c[8] + c[9] * c[9] + c[10] * c[10];
-      a[9] = ia[9];
-      a[10] = p[0] * a[0] * a[1] * a[1];
-      a[11] = p[1] * c[8] + p[2] * c[9] + p[3] * c[10];
-      a[12] = a[10] * p[1];
-      a[13] = a[10] * p[2];
-      a[14] = a[10] * p[3];
-      a[15] = a[12] * a[12] + a[13] * a[13] + a[14] * a[14];
-      a[16] = a[10] - p[4] - c[0];
+      for (int v = 0; v < 8; ++v) prims[v * N + cell] = p[v];
+      for (int v = 0; v < 17; ++v) aux[v * N + cell] = a[v];
+    } else {  // the cell keeps its primitives; finalise reads them
+      atomicAdd((unsigned long long*)&w.counters[2], 1ull);
+      atomicOr((unsigned long long*)&w.counters[3], (unsigned long long)ERR_C2P);
+      for (int v = 1; v < 8; ++v) p[v] = prims[v * N + cell];
+    }
+    double E[3];
+    finalise_e(ideal_weight(g, sigma_of(g, c[0])), p, c + 8, E);
+    for (int v = 0; v < 3; ++v) {
+      cons[(8 + v) * N + cell] = E[v];
+      prims[(8 + v) * N + cell] = E[v];
     }
   }
-  atomicAdd((unsigned long long*)&w.counters[0], 1ull);
-  atomicAdd((unsigned long long*)&w.counters[1], (unsigned long long)evals);
-  if (!ok) {
-    atomicAdd((unsigned long long*)&w.counters[2], 1ull);
-    atomicOr((unsigned long long*)&w.counters[3], (unsigned long long)ERR_C2P);
-    return;
+  const unsigned mask = __ballot_sync(0xffffffffu, active);
+  for (int o = 16; o > 0; o >>= 1) evals += __shfl_down_sync(0xffffffffu, evals, o);
+  if ((threadIdx.x & 31) == 0 && mask) {
+    atomicAdd((unsigned long long*)&w.counters[0], (unsigned long long)__popc(mask));
+    atomicAdd((unsigned long long*)&w.counters[1], (unsigned long long)evals);
   }
-  for (int v = 0; v < 11; ++v) prims[v * N + cell] = p[v];
-  for (int v = 0; v < 17; ++v) aux[v * N + cell] = a[v];
 }
 
-// Hybrid::finalise (hybrid.cc:474-503) on interior cells (the boundary
-// conditions that follow overwrite the ghosts): E blended towards -v x B.
+// Hybrid::finalise on interior cells, after the mixed form's recovery (the
+// boundary conditions that follow overwrite the ghosts).
 __global__ void __launch_bounds__(kThreads)
     k_hybrid_finalise(Grid g, double* cons, double* prims) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -123,16 +155,13 @@ __global__ void __launch_bounds__(kThreads)
   int i, j, k;
   interior_ijk(g, t, i, j, k);
   const long long N = g.Ntot, cell = cell_id(g, i, j, k);
-  const double iW = ideal_weight(g, sigma_of(g, cons[cell]));
-  const double p1 = prims[1 * N + cell], p2 = prims[2 * N + cell], p3 = prims[3 * N + cell];
-  const double p5 = prims[5 * N + cell], p6 = prims[6 * N + cell], p7 = prims[7 * N + cell];
-  const double iE[3] = {-(p2 * p7 - p3 * p6), -(p3 * p5 - p1 * p7), -(p1 * p6 - p2 * p5)};
+  double p[8], c[3], E[3];
+  for (int v = 1; v < 8; ++v) p[v] = prims[v * N + cell];
+  for (int v = 0; v < 3; ++v) c[v] = cons[(8 + v) * N + cell];
+  finalise_e(ideal_weight(g, sigma_of(g, cons[cell])), p, c, E);
   for (int v = 0; v < 3; ++v) {
-    double e = cons[(8 + v) * N + cell];
-    e *= (1 - iW);
-    e += iW * iE[v];
-    cons[(8 + v) * N + cell] = e;
-    prims[(8 + v) * N + cell] = e;
+    cons[(8 + v) * N + cell] = E[v];
+    prims[(8 + v) * N + cell] = E[v];
   }
 }
 
@@ -154,6 +183,39 @@ __global__ void __launch_bounds__(kThreads)
   srmhd::source(ic, g.cp, is);
   for (int v = 0; v < 8; ++v) src[v * N + cell] = iW * is[v] + (1 - iW) * rs[v];
   for (int v = 8; v < 14; ++v) src[v * N + cell] = (1 - iW) * rs[v];
+}
+
+// The half source step of RKSplit2 with a constant conductivity in one pass:
+// cons += h S, S = Hybrid::sourceTermSingleCell (+ S_REGIME w mask when EXT),
+// the expressions of k_hybrid_source, k_hybrid_regime_add and k_add_scaled in
+// their order.  A constant conductivity makes the mask of Hybrid::setMasks one
+// comparison (interior cells lie inside its index ranges, as Ng >= 3), and no
+// cell reads a neighbour's cons, so the update can be in place; with
+// functionalSigma the mask reads neighbours' D and the separate passes stay.
+// Bound by memory: it moves 14 cons planes in and out, 3 aux and 9 extension
+// planes, 40 in all, where the three passes moved 31 + 27 + 42.
+template <bool EXT>
+__global__ void __launch_bounds__(kThreads)
+    k_hybrid_source_add(Grid g, double* cons, const double* __restrict__ aux,
+                        const double* __restrict__ ext, double h) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= n_interior(g)) return;
+  int i, j, k;
+  interior_ijk(g, t, i, j, k);
+  const long long N = g.Ntot, cell = cell_id(g, i, j, k);
+  double c[14], a[17], is[9], rs[14];
+  for (int v = 0; v < 14; ++v) c[v] = cons[v * N + cell];
+  for (int v = 4; v < 7; ++v) a[v] = aux[v * N + cell];
+  const double iW = ideal_weight(g, g.sigma);
+  const int mask = g.sigma > g.sigma_cross - g.sigma_span;
+  srrmhd::source(c, a, g.cp, rs);
+  const double ic[9] = {0, 0, 0, 0, 0, 0, 0, 0, c[12]};
+  srmhd::source(ic, g.cp, is);
+  for (int v = 0; v < 14; ++v) {
+    double src = v < 8 ? iW * is[v] + (1 - iW) * rs[v] : (1 - iW) * rs[v];
+    if (EXT && v < 9) src = src + ext[v * N + cell] * iW * mask;
+    cons[v * N + cell] = c[v] + h * src;
+  }
 }
 
 // Data::sigmaFunc with cell indices (simData.cc:114-127) as Hybrid::setMasks
@@ -254,12 +316,8 @@ cudaError_t launch_hybrid_split(const Grid& g, const double* cons, const double*
 cudaError_t launch_c2p_hybrid(const Grid& g, const double* cons, const double* prims_guess,
                               const double* aux_guess, double* prims, double* aux, C2PWork w,
                               cudaStream_t st) {
-  k_hybrid_c2p<<<blocks_for(n_interior_host(g)), kThreads, 0, st>>>(g, cons, prims_guess,
-                                                                    aux_guess, prims, aux, w);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_hybrid_finalise<<<blocks_for(n_interior_host(g)), kThreads, 0, st>>>(g, const_cast<double*>(cons),
-                                                                         prims);
+  k_hybrid_c2p<<<blocks_for(n_interior_host(g)), kThreads, 0, st>>>(
+      g, const_cast<double*>(cons), prims_guess, aux_guess, prims, aux, w);
   return cudaGetLastError();
 }
 
@@ -279,6 +337,20 @@ cudaError_t launch_hybrid_source(const Grid& g, int order, const double* cons,
   if ((e = launch_regime_ext(g, order, cons, prims, *regime, ext, mixed, st)) != cudaSuccess)
     return e;
   k_hybrid_regime_add<<<blocks_for(nI), kThreads, 0, st>>>(g, cons, ext, src);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_hybrid_source_add(const Grid& g, int order, double* cons, const double* prims,
+                                     const double* aux, const RegimeWork* regime, double* ext,
+                                     bool mixed, double h, cudaStream_t st) {
+  const int b = blocks_for(n_interior_host(g));
+  if (!regime) {
+    k_hybrid_source_add<false><<<b, kThreads, 0, st>>>(g, cons, aux, nullptr, h);
+    return cudaGetLastError();
+  }
+  cudaError_t e = launch_regime_ext(g, order, cons, prims, *regime, ext, mixed, st);
+  if (e != cudaSuccess) return e;
+  k_hybrid_source_add<true><<<b, kThreads, 0, st>>>(g, cons, aux, ext, h);
   return cudaGetLastError();
 }
 

@@ -78,6 +78,10 @@ cudaError_t launch_hybrid_source(const Grid& g, int order, const double* cons,
                                  const double* prims, const double* aux, double* src,
                                  const RegimeWork* regime, double* ext, bool mixed,
                                  cudaStream_t st);
+// The same with a constant conductivity, added in place: cons += h S.
+cudaError_t launch_hybrid_source_add(const Grid& g, int order, double* cons, const double* prims,
+                                     const double* aux, const RegimeWork* regime, double* ext,
+                                     bool mixed, double h, cudaStream_t st);
 cudaError_t launch_hybrid_blend(const Grid& g, double* cons, double* prims, double* aux,
                                 const double* icons, const double* iaux, cudaStream_t st);
 // cons += h src on interior cells.

@@ -157,3 +157,38 @@ def test_mixed_form_against_plain(case):
     l1 = np.abs(out["mixed"] - out["fp64"]).sum() / np.abs(out["fp64"]).sum()
     assert np.all(np.isfinite(out["mixed"]))
     assert l1 < 1e-6, l1
+
+
+@pytest.mark.parametrize("nx,ny,nz,use_regime",
+                         [(33, 0, 0, True), (8, 33, 0, True), (41, 70, 0, True),
+                          (41, 70, 0, False), (9, 8, 10, False)])
+@pytest.mark.parametrize("sigma", [90.0, 120.0, 170.0, 220.0])
+def test_constant_conductivity_one_pass_source(nx, ny, nz, use_regime, sigma):
+    """A constant conductivity takes the one-pass source step, a functional
+    one the separate passes; sigma * D^0 is the same conductivity, so both
+    give the same bits (resistive, blended below and above the crossover, ideal)."""
+    import method_b200 as mb
+    rng = np.random.default_rng(7)
+    cfg = dict(model="hybrid", integrator="rksplit2", nx=nx, ny=ny, nz=nz, xmin=0.0, xmax=1.0,
+               ymin=0.0, ymax=1.0, zmin=0.0, zmax=1.0, endTime=1.0, cfl=0.3, Ng=4,
+               gamma=4.0 / 3.0, sigma=sigma, weno=3, bcs="periodic", useREGIME=use_regime)
+    out = []
+    for functional in (False, True):
+        sim = mb.Simulation(functionalSigma=functional, gam=0.0, **cfg)
+        if not out:
+            p = np.zeros(sim.shape(11))
+            p[0] = 1.0 + 0.1 * rng.random(p.shape[1:])
+            p[1:4] = 0.1 * (rng.random((3,) + p.shape[1:]) - 0.5)
+            p[4] = 1.0
+            p[5:8] = 0.3 * (rng.random((3,) + p.shape[1:]) - 0.5)
+            p[8] = -(p[2] * p[7] - p[3] * p[6])
+            p[9] = -(p[3] * p[5] - p[1] * p[7])
+            p[10] = -(p[1] * p[6] - p[2] * p[5])
+        sim.set_prims(p)
+        sim.step(1e-3)
+        sim.step(1e-3)
+        out.append(sim.state())
+        sim.close()
+    for one, passes in zip(*out):
+        assert np.all(np.isfinite(one))
+        assert np.array_equal(one, passes)
