@@ -6,6 +6,7 @@
 Translation units and their floating-point contracts:
   kernels_fp64.cu   -fmad=false: the plain FP64 form must round every
                     expression like the reference's x86-64 build (no FMA).
+  imex_fp64.cu      -fmad=false: the plain form's implicit IMEX stages.
   regime.cu         -fmad=false: the REGIME source extension, plain form.
   regime_mixed.cu   FMA allowed: its fused tile with FP32 stiff-flux WENO.
   hybrid.cu         -fmad=false: the Hybrid model (blended SRMHD / SRRMHD).
@@ -36,6 +37,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 
 UNITS = [
     ("kernels_fp64.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("imex_fp64.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("regime.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("hybrid.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("regime_mixed.cu", []),

@@ -46,7 +46,7 @@ __device__ __forceinline__ R weno_point(const R* v, int stride) {
   return R(0);
 }
 
-template <int ORDER, typename R>
+template <int ORDER, typename R, bool PAIR = true>
 __device__ __forceinline__ R weno_face(const R* p, const R* m, int stride, int base) {
   // p, m point at the first stencil cell of the region column; `base` is the
   // region index of cell i-H for face i (face between cells i-1 and i).
@@ -59,8 +59,7 @@ __device__ __forceinline__ R weno_face(const R* p, const R* m, int stride, int b
   } else if constexpr (ORDER == 3) {
     // upwind cells i-2, i-1, i ; downwind cells i+1, i, i-1 (weno.cc:123-164)
     if constexpr (sizeof(R) == 8) {
-      return weno3_exact(p[(base + 0) * stride], p[(base + 1) * stride], p[(base + 2) * stride]) +
-             weno3_exact(m[(base + 3) * stride], m[(base + 2) * stride], m[(base + 1) * stride]);
+      return weno_face_exact<3, PAIR>(p + base * stride, m + (base + 3) * stride, stride);
     } else {
       const float2 r = weno3_fast2(make_float2(p[(base + 0) * stride], m[(base + 3) * stride]),
                                    make_float2(p[(base + 1) * stride], m[(base + 2) * stride]),
@@ -70,10 +69,7 @@ __device__ __forceinline__ R weno_face(const R* p, const R* m, int stride, int b
   } else {
     // upwind cells i-3 .. i+1 ; downwind cells i+2 .. i-2 (weno.cc:175-228)
     if constexpr (sizeof(R) == 8) {
-      return weno5_exact(p[(base + 0) * stride], p[(base + 1) * stride], p[(base + 2) * stride],
-                         p[(base + 3) * stride], p[(base + 4) * stride]) +
-             weno5_exact(m[(base + 5) * stride], m[(base + 4) * stride], m[(base + 3) * stride],
-                         m[(base + 2) * stride], m[(base + 1) * stride]);
+      return weno_face_exact<5, PAIR>(p + base * stride, m + (base + 5) * stride, stride);
     } else {
       const float2 r = weno5_fast2(make_float2(p[(base + 0) * stride], m[(base + 5) * stride]),
                                    make_float2(p[(base + 1) * stride], m[(base + 4) * stride]),
@@ -143,18 +139,22 @@ __device__ __forceinline__ void split_cell(const Grid& g, const double* __restri
   }
 }
 
-// Flux difference of one cell along one direction, f_right / d - f_left / d
-// (fluxVectorSplitting.cc:105-111): exactly so in FP64; in the FP32 form
-// through one reciprocal of the cell size.
+// A face's flux over the cell size: the flux difference of a cell is
+// f_right / d - f_left / d (fluxVectorSplitting.cc:105-111), so the division
+// is done once per face and the cells on both sides subtract.  FP64: the
+// IEEE quotient; FP32: one reciprocal of the cell size.
 template <typename R>
-__device__ __forceinline__ R face_diff(R right, R left, R d) {
-  if constexpr (sizeof(R) == 8) {
-    return right / d - left / d;
-  } else {
-    const R inv = R(1) / d;
-    return right * inv - left * inv;
-  }
-}
+struct FaceScale;
+template <>
+struct FaceScale<double> : Divisor {
+  using Divisor::Divisor;
+};
+template <>
+struct FaceScale<float> {
+  float inv;
+  __device__ __forceinline__ explicit FaceScale(float d) : inv(1.0f / d) {}
+  __device__ __forceinline__ float operator()(float x) const { return x * inv; }
+};
 
 // The stage's output for one interior cell from its flux difference `acc`
 // (fnet of FVS::F): fnet itself, the Euler step U - dt fnet, the RK2
@@ -239,13 +239,14 @@ __device__ __forceinline__ void fvs2d_tile(const Grid& g, const double* __restri
     split_cell<M, R>(g, cons, prims, aux, mapped_cell(g, gi, gj, 0), 0, sp + e, sm + e, S::RX);
   }
   __syncthreads();
+  const FaceScale<R> over_dx(R(g.dx)), over_dy(R(g.dy));
   // Item e = (v, fi, lane): a step of NT items is TI rows of faces, so the
   // lane stays fixed and (v, fi) advance without a division.
   for (int e = tid, v = 0, fi = ty; e < NC * S::FX; e += NT) {
     const R* P = sp + v * S::RX + lane;
     const R* Mm = sm + v * S::RX + lane;
     // face i0+fi: cell i-H sits at region row fi
-    sr[e] = weno_face<ORDER, R>(P, Mm, TJ, fi);
+    sr[e] = over_dx(weno_face<ORDER, R>(P, Mm, TJ, fi));
     fi += TI;
     if (fi > TI) {
       fi -= TI + 1;
@@ -253,13 +254,9 @@ __device__ __forceinline__ void fvs2d_tile(const Grid& g, const double* __restri
     }
   }
   __syncthreads();
-  {
-    const R dx = R(g.dx);
 #pragma unroll
-    for (int v = 0; v < NC; ++v)
-      acc[v] = face_diff<R>(sr[v * S::FX + (ty + 1) * TJ + lane], sr[v * S::FX + ty * TJ + lane],
-                            dx);
-  }
+  for (int v = 0; v < NC; ++v)
+    acc[v] = sr[v * S::FX + (ty + 1) * TJ + lane] - sr[v * S::FX + ty * TJ + lane];
   __syncthreads();
 
   // ---------------- y direction ----------------
@@ -279,7 +276,7 @@ __device__ __forceinline__ void fvs2d_tile(const Grid& g, const double* __restri
     for (int e = tid; e < NC * S::FY; e += NT) {
       const R* P = sp + v * S::RY + r * WY;
       const R* Mm = sm + v * S::RY + r * WY;
-      sr[e] = weno_face<ORDER, R>(P, Mm, 1, fj);
+      sr[e] = over_dy(weno_face<ORDER, R>(P, Mm, 1, fj));
       fj += FS;
       r += RS;
       if (fj > TJ) {
@@ -294,11 +291,10 @@ __device__ __forceinline__ void fvs2d_tile(const Grid& g, const double* __restri
   }
   __syncthreads();
   if (ci < g.ie && cj < g.je) {
-    const R dy = R(g.dy);
 #pragma unroll
     for (int v = 0; v < NC; ++v)
-      acc[v] = acc[v] + face_diff<R>(sr[v * S::FY + ty * (TJ + 1) + lane + 1],
-                                     sr[v * S::FY + ty * (TJ + 1) + lane], dy);
+      acc[v] = acc[v] + (sr[v * S::FY + ty * (TJ + 1) + lane + 1] -
+                         sr[v * S::FY + ty * (TJ + 1) + lane]);
 
     stage_update<M, R>(g, cons, aux, u0, out, dt, mode, tail, cell_id(g, ci, cj, 0), acc);
   }

@@ -66,8 +66,10 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
                            S::RX);
   }
   __syncthreads();
+  const Divisor over_dx(g.dx);
   for (int e = tid, v = 0, fi = ty; e < NV * S::FX; e += NT) {
-    sr[e] = weno_face<ORDER, double>(sp + v * S::RX + lane, sm + v * S::RX + lane, TJ, fi);
+    sr[e] = over_dx(
+        weno_face<ORDER, double, false>(sp + v * S::RX + lane, sm + v * S::RX + lane, TJ, fi));
     fi += TI;
     if (fi > TI) {
       fi -= TI + 1;
@@ -77,8 +79,7 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
   __syncthreads();
 #pragma unroll
   for (int v = 0; v < NV; ++v)
-    acc[V0 + v] = face_diff<double>(sr[v * S::FX + (ty + 1) * TJ + lane],
-                                    sr[v * S::FX + ty * TJ + lane], g.dx);
+    acc[V0 + v] = sr[v * S::FX + (ty + 1) * TJ + lane] - sr[v * S::FX + ty * TJ + lane];
   __syncthreads();
 
   // y direction: region columns j0-H .. j0+TJ+H-1
@@ -91,10 +92,12 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
   }
   __syncthreads();
   {
+    const Divisor over_dy(g.dy);
     constexpr int RS = NT / (TJ + 1), FS = NT % (TJ + 1);
     int v = 0, r = tid / (TJ + 1), fj = tid % (TJ + 1);
     for (int e = tid; e < NV * S::FY; e += NT) {
-      sr[e] = weno_face<ORDER, double>(sp + v * S::RY + r * WY, sm + v * S::RY + r * WY, 1, fj);
+      sr[e] = over_dy(
+          weno_face<ORDER, double, false>(sp + v * S::RY + r * WY, sm + v * S::RY + r * WY, 1, fj));
       fj += FS;
       r += RS;
       if (fj > TJ) {
@@ -110,8 +113,8 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
   __syncthreads();
 #pragma unroll
   for (int v = 0; v < NV; ++v)
-    acc[V0 + v] = acc[V0 + v] + face_diff<double>(sr[v * S::FY + ty * (TJ + 1) + lane + 1],
-                                                  sr[v * S::FY + ty * (TJ + 1) + lane], g.dy);
+    acc[V0 + v] = acc[V0 + v] + (sr[v * S::FY + ty * (TJ + 1) + lane + 1] -
+                                 sr[v * S::FY + ty * (TJ + 1) + lane]);
   __syncthreads();
   if constexpr (Q + 1 < Fvs2dGroupSmem<M, ORDER, TI, G>::NG)
     group_pass<M, ORDER, TI, G, Q + 1>(g, cons, prims, aux, i0, j0, acc, smem_raw);

@@ -1,0 +1,76 @@
+"""The plain form's WENO3/5 weights and face scaling divide without branches
+where the operands allow it (csrc/div64.cuh) and by IEEE division elsewhere;
+both must give the bits of the oracle (oracle/oracle.c, plain C), in the
+generic path and in both fused tiles, at ragged tile edges."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+G = 4.0 / 3.0
+
+
+def config(nx, ny, nz=0, weno=5, bcs="periodic"):
+    return dict(model="srmhd", nx=nx, ny=ny, nz=nz, xmin=0.0, xmax=1.0, ymin=0.0, ymax=1.3,
+                zmin=0.0, zmax=0.7, endTime=1.0, cfl=0.3, Ng=4, gamma=G, weno=weno, bcs=bcs,
+                integrator="rk2")
+
+
+@pytest.mark.parametrize("weno", [3, 5])
+@pytest.mark.parametrize("nx,ny,nz", [(40, 0, 0), (9, 33, 0), (6, 7, 5)])
+@pytest.mark.parametrize("scale", [1.0, 1e-9, 1e-140, 1e66, 1e67, 1e130])
+def test_flux_of_any_size_matches_oracle(weno, nx, ny, nz, scale):
+    """FVS::F of states whose smoothness indicators are zero (constant
+    regions), ordinary, beyond the branch-free range (indicators above 2^448)
+    and around its edge."""
+    import method_b200 as mb
+    from oracle import port
+    cfg = config(nx, ny, nz, weno)
+    rng = np.random.default_rng(3)
+    sim = mb.Simulation(**cfg)
+    p, c, a = (sim.zeros(n) for n in (sim.Nprims, sim.Ncons, sim.Naux))
+    c[:] = scale * (rng.random(c.shape) - 0.5)
+    c[:, : c.shape[1] // 3] = scale  # constant: every indicator is exactly zero
+    c[3] = 0.0
+    p[1:4] = 0.6 * (rng.random(p[1:4].shape) - 0.5)
+    p[4] = scale * rng.random(p[4].shape)
+    p[5:7] = rng.random(p[5:7].shape) - 0.5
+    a[1] = 1.0 + rng.random(a[1].shape)
+    a[4:9] = rng.random(a[4:9].shape) - 0.5
+    sim.upload(c, p, a)
+    got = sim.flux_F()
+    sim.close()
+    safe = p.copy()
+    safe[0], safe[4] = 1.0, 1.0
+    o = port.PortSim(safe, **cfg)
+    want = o.flux_F(c, p, a)
+    o.close()
+    assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("weno", [3, 5])
+@pytest.mark.parametrize("nx,ny", [(8, 32), (7, 31), (9, 33), (17, 70), (100, 736)])
+@pytest.mark.parametrize("bcs", ["periodic", "outflow"])
+def test_fused_step_matches_oracle(weno, nx, ny, bcs):
+    """One RK2 step of a blast with constant regions, by the one-pass tile and,
+    at 100 x 736 (299 tiles), by the grouped one."""
+    import method_b200 as mb
+    from oracle import port
+    cfg = config(nx, ny, 0, weno, bcs)
+    sim = mb.Simulation(**cfg)
+    p = sim.zeros(sim.Nprims)
+    X, Y = np.meshgrid(np.linspace(0, 1, sim.Nx), np.linspace(0, 1, sim.Ny), indexing="ij")
+    hot = ((X - 0.5) ** 2 + (Y - 0.4) ** 2 < 0.06)[:, :, None]
+    p[0] = np.where(hot, 1.0, 0.1)
+    p[4] = np.where(hot, 10.0, 0.05)
+    p[1] = 0.3 * np.sin(7 * Y)[:, :, None]
+    p[5], p[6] = 0.2, 0.1 * np.cos(5 * X)[:, :, None]
+    sim.set_prims(p)
+    o = port.PortSim(p, **cfg)
+    dt = 0.05 / max(nx, ny)
+    sim.step(dt)
+    o.step_dt(dt)
+    for name, got, want in zip(("cons", "prims", "aux"), sim.state(), o.state()):
+        assert np.array_equal(got, want), name
+    sim.close()
+    o.close()
