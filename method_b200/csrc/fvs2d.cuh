@@ -300,14 +300,225 @@ __device__ __forceinline__ void fvs2d_tile(const Grid& g, const double* __restri
   }
 }
 
+// The FP32 tiles of WENO3/5 work on pairs of variables: f+-, and the faces are
+// kept in shared memory as (variable 2q, variable 2q + 1), so that one 8-byte
+// access moves two variables and both lanes of the FP32x2 reconstruction do
+// useful work; an odd last variable pairs its upwind with its downwind side.
+//
+// f+ and f- of a region of RSZ cells.
+template <class M, int ORDER, int RSZ>
+struct SplitRegion {
+  static constexpr int NC = M::NC, NP = NC / 2;
+  static constexpr bool ODD = NC % 2;
+  static constexpr size_t bytes = sizeof(float) * (size_t)(2 * NC * RSZ);
+  float2 *sp, *sm;  // [NP][RSZ]
+  float *op, *om;   // the odd variable's
+  __device__ __forceinline__ explicit SplitRegion(unsigned char* raw) {
+    sp = reinterpret_cast<float2*>(raw);
+    sm = sp + NP * RSZ;
+    op = reinterpret_cast<float*>(sm + NP * RSZ);
+    om = op + RSZ;
+  }
+
+  // f+- = 0.5 (f +- U) of one cell along `dir` into slot e (the values of
+  // fluxVectorSplitting.cc:22-33 in FP32: halving is exact).
+  __device__ __forceinline__ void split(const Grid& g, const double* __restrict__ cons,
+                                        const double* __restrict__ prims,
+                                        const double* __restrict__ aux, long long cell, int dir,
+                                        int e) const {
+    float c[M::NC], p[M::NP], a[M::NA], f[NC];
+    M::template load_flux_inputs<float>(cons, prims, aux, g.Ntot, cell, c, p, a);
+    M::template flux_g<float>(g, c, p, a, dir, f);
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      const float2 fv = make_float2(f[2 * q], f[2 * q + 1]);
+      const float2 cv = make_float2(c[2 * q], c[2 * q + 1]);
+      sp[q * RSZ + e] = __ffma2_rn(fv, f2(0.5f), __fmul2_rn(cv, f2(0.5f)));
+      sm[q * RSZ + e] = __ffma2_rn(fv, f2(0.5f), __fmul2_rn(cv, f2(-0.5f)));
+    }
+    if constexpr (ODD) {
+      const float2 h =
+          __ffma2_rn(f2(f[NC - 1]), f2(0.5f), __fmul2_rn(f2(c[NC - 1]), make_float2(0.5f, -0.5f)));
+      op[e] = h.x;
+      om[e] = h.y;
+    }
+  }
+
+  // Pair q at the face whose upwind stencil starts at slot b, cells st
+  // apart, over the cell size.
+  __device__ __forceinline__ float2 face(int q, int b, int st, float inv) const {
+    const float2* P = sp + q * RSZ + b;
+    const float2* Q = sm + q * RSZ + b;
+    float2 u, d;
+    if constexpr (ORDER == 3) {
+      u = weno3_fast2(P[0], P[st], P[2 * st]);
+      d = weno3_fast2(Q[3 * st], Q[2 * st], Q[st]);
+    } else {
+      u = weno5_fast2(P[0], P[st], P[2 * st], P[3 * st], P[4 * st]);
+      d = weno5_fast2(Q[5 * st], Q[4 * st], Q[3 * st], Q[2 * st], Q[st]);
+    }
+    return __fmul2_rn(__fadd2_rn(u, d), f2(inv));
+  }
+  __device__ __forceinline__ float face_odd(int b, int st, float inv) const {
+    return weno_face<ORDER, float>(op + b, om + b, st, 0) * inv;
+  }
+};
+
+// FSZ faces of every variable.
+template <class M, int FSZ>
+struct FaceArray {
+  static constexpr int NC = M::NC, NP = NC / 2;
+  static constexpr bool ODD = NC % 2;
+  static constexpr size_t bytes = sizeof(float) * (size_t)(NC * FSZ);
+  float2* r;
+  float* o;
+  __device__ __forceinline__ explicit FaceArray(unsigned char* raw) {
+    r = reinterpret_cast<float2*>(raw);
+    o = reinterpret_cast<float*>(r + NP * FSZ);
+  }
+  // Every variable of the faces at region slot b: stored at slot e and left
+  // in `own`.
+  template <class S>
+  __device__ __forceinline__ void fill(const S& reg, int b, int st, float inv, int e,
+                                       float* own) const {
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      const float2 v = reg.face(q, b, st, inv);
+      r[q * FSZ + e] = v;
+      own[2 * q] = v.x;
+      own[2 * q + 1] = v.y;
+    }
+    if constexpr (ODD) own[NC - 1] = o[e] = reg.face_odd(b, st, inv);
+  }
+  // diff = (the faces at slot e) - own.
+  __device__ __forceinline__ void minus(int e, const float* own, float* diff) const {
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      const float2 v = r[q * FSZ + e];
+      diff[2 * q] = v.x - own[2 * q];
+      diff[2 * q + 1] = v.y - own[2 * q + 1];
+    }
+    if constexpr (ODD) diff[NC - 1] = o[e] - own[NC - 1];
+  }
+};
+
+// The faces past a tile's own: its last face row in x, one pair (or the odd
+// variable) per warp, and its last face column in y, from the last warp down.
+template <class M, int ORDER, int TI>
+struct LastFaces {
+  using S = Fvs2dSmem<M, float, ORDER, TI>;
+  using Region = SplitRegion<M, ORDER, S::RMAX>;
+  using Faces = FaceArray<M, S::FMAX>;
+  static constexpr int NP = M::NC / 2, TJ = S::TJ, NT = 32 * TI, WY = TJ + 2 * S::H;
+  static constexpr bool ODD = M::NC % 2;
+  static constexpr int K1 = (TI * NP + 31) / 32 * 32;
+  static_assert(K1 + (ODD ? TI : 0) <= NT, "at most one item per thread");
+  __device__ __forceinline__ static void x(const Region& reg, const Faces& F, int lane, int ty,
+                                           float inv) {
+    const int b = TI * TJ + lane;
+    for (int q = ty; q < NP + (ODD ? 1 : 0); q += TI) {
+      if (q < NP)
+        F.r[q * S::FMAX + b] = reg.face(q, b, TJ, inv);
+      else
+        F.o[b] = reg.face_odd(b, TJ, inv);
+    }
+  }
+  __device__ __forceinline__ static void y(const Region& reg, const Faces& F, int tid,
+                                           float inv) {
+    const int k = NT - 1 - tid;
+    if (k < TI * NP) {
+      const int q = k / TI, r = k % TI;
+      F.r[q * S::FMAX + r * (TJ + 1) + TJ] = reg.face(q, r * WY + TJ, 1, inv);
+    } else if (ODD && k >= K1 && k < K1 + TI) {
+      const int r = k - K1;
+      F.o[r * (TJ + 1) + TJ] = reg.face_odd(r * WY + TJ, 1, inv);
+    }
+  }
+};
+
+// FP32 tile, one direction after the other (the phases of fvs2d_tile).  Thread
+// (ty, lane) owns face ty (x) or lane (y) of every pair at constant offsets
+// from one address, keeps its own (left) faces in registers and reads only
+// the right neighbours'; one barrier less than fvs2d_tile.  Bound by the
+// latency of the split's loads and by issue (ncu, OT 512^2 WENO5: 23.4 -> 16.4 M
+// warp instructions a launch, 53% -> 46% issue active): OT 1024^2 0.153 ->
+// 0.130 ms per launch.  Holding the x and the y split at once, so that each
+// cell is loaded 1.9 times and not 2.9, leaves room for 3 CTAs of 74 KB on an
+// SM instead of 4 and was slower (0.150 ms).
+template <class M, int ORDER, int TI>
+__device__ __forceinline__ void fvs2d_tile_pairs(const Grid& g, const double* __restrict__ cons,
+                                                 const double* __restrict__ prims,
+                                                 const double* __restrict__ aux, const double* u0,
+                                                 double* out, double dt, int mode, int ti, int tj,
+                                                 unsigned char* smem_raw, StageTail tail) {
+  using S = Fvs2dSmem<M, float, ORDER, TI>;
+  using Region = SplitRegion<M, ORDER, S::RMAX>;
+  using Faces = FaceArray<M, S::FMAX>;
+  using Last = LastFaces<M, ORDER, TI>;
+  constexpr int NC = M::NC, TJ = S::TJ, H = S::H, NT = 32 * TI, WY = TJ + 2 * H;
+  const Region reg(smem_raw);
+  const Faces F(smem_raw + Region::bytes);
+  const int lane = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + lane;
+  const int i0 = g.is + ti * TI, j0 = g.js + tj * TJ;
+  const int ci = i0 + ty, cj = j0 + lane;
+  if (ci < g.ie && cj < g.je) prefetch_tail<M>(g, u0, mode, tail, cell_id(g, ci, cj, 0));
+  float acc[NC], own[NC];
+
+  // ---------------- x direction ----------------
+  for (int e = tid; e < S::RX; e += NT) {
+    const int gi = min(i0 - H + e / TJ, g.ie - 1 + H), gj = min(j0 + e % TJ, g.je - 1);
+    reg.split(g, cons, prims, aux, mapped_cell(g, gi, gj, 0), 0, e);
+  }
+  __syncthreads();
+  {
+    const float inv = 1.0f / float(g.dx);
+    const int b = ty * TJ + lane;
+    F.fill(reg, b, TJ, inv, b, own);
+    Last::x(reg, F, lane, ty, inv);
+    __syncthreads();
+    F.minus(b + TJ, own, acc);
+  }
+
+  // ---------------- y direction (the x split is dead since the barrier) ------
+  for (int e = tid; e < S::RY; e += NT) {
+    const int gi = min(i0 + e / WY, g.ie - 1), gj = min(j0 - H + e % WY, g.je - 1 + H);
+    reg.split(g, cons, prims, aux, mapped_cell(g, gi, gj, 0), 1, e);
+  }
+  __syncthreads();
+  const float inv = 1.0f / float(g.dy);
+  const int o = ty * (TJ + 1) + lane;
+  F.fill(reg, ty * WY + lane, 1, inv, o, own);
+  Last::y(reg, F, tid, inv);
+  __syncthreads();
+  if (ci >= g.ie || cj >= g.je) return;
+  float dy[NC];
+  F.minus(o + 1, own, dy);
+#pragma unroll
+  for (int v = 0; v < NC; ++v) acc[v] = acc[v] + dy[v];
+  stage_update<M, float>(g, cons, aux, u0, out, dt, mode, tail, cell_id(g, ci, cj, 0), acc);
+}
+
+// The stage's tile in the form that serves R and ORDER.
+template <class M, typename R, int ORDER, int TI>
+__device__ __forceinline__ void fvs2d_any_tile(const Grid& g, const double* __restrict__ cons,
+                                               const double* __restrict__ prims,
+                                               const double* __restrict__ aux, const double* u0,
+                                               double* out, double dt, int mode, int ti, int tj,
+                                               unsigned char* smem_raw, StageTail tail) {
+  if constexpr (sizeof(R) == 4 && ORDER <= 5)
+    fvs2d_tile_pairs<M, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti, tj, smem_raw, tail);
+  else
+    fvs2d_tile<M, R, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti, tj, smem_raw, tail);
+}
+
 template <class M, typename R, int ORDER, int TI>
 __global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, R, ORDER, TI>()))
     k_fvs2d(Grid g, const double* __restrict__ cons, const double* __restrict__ prims,
             const double* __restrict__ aux, const double* u0, double* out, double dt,
             int mode, StageTail tail, int ti0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  fvs2d_tile<M, R, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti0 + blockIdx.y,
-                              blockIdx.x, smem_raw, tail);
+  fvs2d_any_tile<M, R, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti0 + blockIdx.y,
+                                  blockIdx.x, smem_raw, tail);
 }
 
 }  // namespace mth

@@ -786,9 +786,9 @@ __global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, float, ORDER, TI
     const Item w = items[it];
     const Member& d = mem[w.m];
     const Grid g = d.g;
-    fvs2d_tile<M, float, ORDER, TI>(g, d.a[ic], d.a[ip], d.a[ia], iu0 >= 0 ? d.a[iu0] : nullptr,
-                                    d.a[iout], d.dt, mode, w.a, w.b, smem_raw,
-                                    StageTail{d.a[EA_F1], d.a[EA_S1], g.cp});
+    fvs2d_any_tile<M, float, ORDER, TI>(g, d.a[ic], d.a[ip], d.a[ia],
+                                        iu0 >= 0 ? d.a[iu0] : nullptr, d.a[iout], d.dt, mode, w.a,
+                                        w.b, smem_raw, StageTail{d.a[EA_F1], d.a[EA_S1], g.cp});
     __syncthreads();
   }
 }

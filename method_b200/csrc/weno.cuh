@@ -177,51 +177,63 @@ __device__ __forceinline__ double weno_face_exact(const double* p, const double*
   return u + d + 0.0;  // + 0.0: a zero face value is +0, as the reference's sums from zero give
 }
 
-// FP32 forms: the upwind (.x) and downwind (.y) reconstructions of one face
-// in FP32x2 arithmetic (sm_100 __ffma2_rn / __fadd2_rn / __fmul2_rn: one
-// instruction for both sides, each lane rounded as the scalar operation).
-// Linear weights are taken times 3 (WENO3) and times 10 (WENO5), and the
-// WENO5 Jiang-Shu indicators times 4, 13/3 (a - 2b + c)^2 + (.)^2, with eps
-// times 16: none of these scalings changes the normalised weights.
+// FP32 forms: two reconstructions at once in FP32x2 arithmetic (sm_100
+// __ffma2_rn / __fadd2_rn / __fmul2_rn: one instruction for both lanes, each
+// rounded as the scalar operation) -- two variables of one side of a face, or
+// the upwind (.x) and downwind (.y) sides of one variable.
 //
-// One reciprocal per side: with q_k = eps + beta_k^2 the weights
-// (d_k / q_k) / sum_j (d_j / q_j) equal d_k P_k / sum_j d_j P_j with P_k the
-// product of the other stencils' q (WENO5; for WENO3 simply the other q), so
-// only the final normalisation divides.  WENO5 first scales the three q by
-// the power of two that brings the largest into [1, 2) (exponent bits only,
-// exact), so the products neither overflow for large flux jumps nor
-// underflow below the largest weight's scale.
+// In first differences d_k = v_{k+1} - v_k and second ones t_k = d_{k+1} - d_k
+// the Jiang-Shu indicators (times 4) are 13/3 t^2 + u^2 with u_0 = t_0 + 2 d_1,
+// u_1 = d_1 + d_2, u_2 = t_2 - 2 d_2, and the face value is v_2 plus the weighted
+// corrections d_1/2 + t_0/3, d_2/2 - t_1/6, d_2/2 - t_2/6.  With q_k = eps +
+// beta_k^2 (eps times 16) the weights (c_k / q_k) / sum_j (c_j / q_j), c = 1 : 6 : 3,
+// equal c_k P_k / sum_j c_j P_j with P_k the product of the other two q, so only
+// the final normalisation divides.  The q are first scaled by the power of two
+// that brings their sum into [2^30, 2^31) (exponent bits only, exact): the
+// products then neither overflow nor fall out of the normal range, for
+// jumps up to where beta^2 itself overflows, so an approximate reciprocal
+// without subnormal handling serves.  (WENO3's two weights are normalised before
+// they meet the differences, which serves as well.)
+// 47 instructions a pair of points, 59 before in the form with separate
+// stencil sums and maximum-based scaling.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 
+__device__ __forceinline__ float rcp_normal(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ float2 rcp2(float2 q) {
-  return make_float2(__fdividef(1.0f, q.x), __fdividef(1.0f, q.y));
+  return make_float2(rcp_normal(q.x), rcp_normal(q.y));
 }
 
-// 2^-floor(log2 m) for a positive normal m below 2^126, from the exponent bits.
-__device__ __forceinline__ float pow2_inv(float m) {
-  return __int_as_float(0x7F000000 - (__float_as_int(m) & 0x7F800000));
+// 2^(30 - floor(log2 s)) for a normal s of at least 2^-90, from the exponent bits.
+__device__ __forceinline__ float pow2_scale(float s) {
+  return __uint_as_float(0x8E000000u - (__float_as_uint(s) & 0x7F800000u));
 }
 
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  return __ffma2_rn(f2(-1.0f), b, a);
+}
+
+// v_1 + (q_1 / Q) d_0 / 2 + (q_0 / Q) d_1, Q = q_1 + 2 q_0: linear weights 1 : 2.
 __device__ __forceinline__ float2 weno3_fast2(float2 v0, float2 v1, float2 v2) {
-  const float2 d0 = __ffma2_rn(f2(-1.0f), v0, v1), d1 = __ffma2_rn(f2(-1.0f), v1, v2);
+  const float2 d0 = sub2(v1, v0), d1 = sub2(v2, v1);
   const float2 b0 = __fmul2_rn(d0, d0), b1 = __fmul2_rn(d1, d1);
   const float2 q0 = __ffma2_rn(b0, b0, f2(1e-16f)), q1 = __ffma2_rn(b1, b1, f2(1e-16f));
-  const float2 s0 = __ffma2_rn(f2(1.5f), v1, __fmul2_rn(f2(-0.5f), v0));
-  const float2 s1 = __fmul2_rn(f2(0.5f), __fadd2_rn(v2, v1));
-  // weights 1/q0 : 2/q1  =  q1 : 2 q0
-  const float2 a1 = __fmul2_rn(f2(2.0f), q0);
-  const float2 num = __ffma2_rn(q1, s0, __fmul2_rn(a1, s1));
-  return __fmul2_rn(num, rcp2(__fadd2_rn(q1, a1)));
+  const float2 r = rcp2(__ffma2_rn(f2(2.0f), q0, q1));
+  return __ffma2_rn(__fmul2_rn(q1, r), __fmul2_rn(f2(0.5f), d0),
+                    __ffma2_rn(__fmul2_rn(q0, r), d1, v1));
 }
 
 __device__ __forceinline__ float2 weno5_fast2(float2 v0, float2 v1, float2 v2, float2 v3,
                                               float2 v4) {
-  const float2 t0 = __fadd2_rn(__ffma2_rn(f2(-2.0f), v1, v0), v2);
-  const float2 u0 = __ffma2_rn(f2(3.0f), v2, __ffma2_rn(f2(-4.0f), v1, v0));
-  const float2 t1 = __fadd2_rn(__ffma2_rn(f2(-2.0f), v2, v1), v3);
-  const float2 u1 = __ffma2_rn(f2(-1.0f), v3, v1);
-  const float2 t2 = __fadd2_rn(__ffma2_rn(f2(-2.0f), v3, v2), v4);
-  const float2 u2 = __ffma2_rn(f2(3.0f), v2, __ffma2_rn(f2(-4.0f), v3, v4));
+  const float2 d0 = sub2(v1, v0), d1 = sub2(v2, v1), d2 = sub2(v3, v2), d3 = sub2(v4, v3);
+  const float2 t0 = sub2(d1, d0), t1 = sub2(d2, d1), t2 = sub2(d3, d2);
+  const float2 u0 = __ffma2_rn(f2(2.0f), d1, t0);
+  const float2 u1 = __fadd2_rn(d1, d2);
+  const float2 u2 = __ffma2_rn(f2(-2.0f), d2, t2);
   const float2 c13 = f2(13.0f / 3.0f);
   const float2 b0 = __ffma2_rn(__fmul2_rn(c13, t0), t0, __fmul2_rn(u0, u0));
   const float2 b1 = __ffma2_rn(__fmul2_rn(c13, t1), t1, __fmul2_rn(u1, u1));
@@ -229,23 +241,19 @@ __device__ __forceinline__ float2 weno5_fast2(float2 v0, float2 v1, float2 v2, f
   float2 q0 = __ffma2_rn(b0, b0, f2(16e-16f));
   float2 q1 = __ffma2_rn(b1, b1, f2(16e-16f));
   float2 q2 = __ffma2_rn(b2, b2, f2(16e-16f));
-  const float2 sc = make_float2(pow2_inv(fmaxf(fmaxf(q0.x, q1.x), q2.x)),
-                                pow2_inv(fmaxf(fmaxf(q0.y, q1.y), q2.y)));
+  const float2 qs = __fadd2_rn(__fadd2_rn(q0, q1), q2);
+  const float2 sc = make_float2(pow2_scale(qs.x), pow2_scale(qs.y));
   q0 = __fmul2_rn(q0, sc);
   q1 = __fmul2_rn(q1, sc);
   q2 = __fmul2_rn(q2, sc);
-  // linear weights 1 : 6 : 3 (x10) over q0 : q1 : q2, times q0 q1 q2
-  const float2 a0 = __fmul2_rn(q1, q2);
-  const float2 a1 = __fmul2_rn(__fmul2_rn(f2(6.0f), q0), q2);
-  const float2 a2 = __fmul2_rn(__fmul2_rn(f2(3.0f), q0), q1);
-  // candidate stencils at the face, the 1/6 folded into the coefficients
-  const float2 c3 = f2(1.0f / 3.0f), c6 = f2(-1.0f / 6.0f), c56 = f2(5.0f / 6.0f);
-  const float2 s0 = __ffma2_rn(f2(11.0f / 6.0f), v2,
-                               __ffma2_rn(f2(-7.0f / 6.0f), v1, __fmul2_rn(c3, v0)));
-  const float2 s1 = __ffma2_rn(c3, v3, __ffma2_rn(c56, v2, __fmul2_rn(c6, v1)));
-  const float2 s2 = __ffma2_rn(c6, v4, __ffma2_rn(c56, v3, __fmul2_rn(c3, v2)));
-  const float2 num = __ffma2_rn(a0, s0, __ffma2_rn(a1, s1, __fmul2_rn(a2, s2)));
-  return __fmul2_rn(num, rcp2(__fadd2_rn(__fadd2_rn(a0, a1), a2)));
+  const float2 p0 = __fmul2_rn(q1, q2), p1 = __fmul2_rn(q0, q2), p2 = __fmul2_rn(q0, q1);
+  // the corrections times 1, 6, 3
+  const float2 e0 = __ffma2_rn(f2(1.0f / 3.0f), t0, __fmul2_rn(f2(0.5f), d1));
+  const float2 e1 = __ffma2_rn(f2(2.0f), d2, d1);  // 3 d_2 - t_1
+  const float2 e2 = __ffma2_rn(f2(-0.5f), t2, __fmul2_rn(f2(1.5f), d2));
+  const float2 num = __ffma2_rn(p0, e0, __ffma2_rn(p1, e1, __fmul2_rn(p2, e2)));
+  const float2 den = __ffma2_rn(f2(6.0f), p1, __ffma2_rn(f2(3.0f), p2, p0));
+  return __ffma2_rn(num, rcp2(den), v2);
 }
 
 }  // namespace mth
