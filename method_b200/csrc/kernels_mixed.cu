@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "div64.cuh"
 #include "ensemble.h"
 #include "fvs2d.cuh"
 #include "hybrid.cuh"
@@ -30,6 +31,20 @@ namespace mth {
 
 namespace {
 
+// 1/x and 1/sqrt(x) of a normal positive (rcp: or negative) x to about one ulp,
+// without the branches of the library's division and rsqrt: Newton's series
+// from the hardware's approximations, x y0^2 = 1 - e with |e| < 2^-18 (for the
+// root y = y0 (1 + e/2 + 3/8 e^2 + ...); the e^3 term is below 2^-55).  The
+// recoveries are chains of them at 40-48% of the FP64 pipe, bound by the
+// chains' latency.
+__device__ __forceinline__ double rcp64(double x) { return div_rcp(x); }
+__device__ __forceinline__ double rsqrt64(double x) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+  const double e = fma(-(x * y0), y0, 1.0);
+  return fma(y0 * e, fma(0.375, e, 0.5), y0);
+}
+
 // Newton in Z for SRMHD, safeguarded by a bracket.  v^2(Z) above is strictly
 // decreasing for Z > 0, so "v^2 >= 1 or g < 0" marks the left of the root
 // and g > 0 its right; a Newton step that leaves the bracket (or a zero or
@@ -38,16 +53,21 @@ namespace {
 //
 // One division and one reciprocal square root per evaluation: 1/(Z^2 (Z +
 // B^2)^2) also gives 1/Z^2 and 1/Z.
+// RCP: by rcp64 / rsqrt64, else by the library.  The grid recovery's kernels
+// (64 registers) keep the library's: the straight-line forms' longer live
+// ranges made them reload 600 bytes of spills a cell instead of 70 (OT 1024^2
+// step 0.424 against 0.421 ms); the batched recovery, at 80 registers, gains.
+template <bool RCP>
 __device__ __forceinline__ bool srmhd_g(double Z, double D, double tau, double BS2, double Bsq,
                                         double Ssq, double k, double& gv, double& dg,
                                         double& v2) {
   const double Z2 = Z * Z, ZB = Z + Bsq;
-  const double iDn = 1 / (Z2 * ZB * ZB);
+  const double iDn = RCP ? rcp64(Z2 * ZB * ZB) : 1 / (Z2 * ZB * ZB);
   v2 = fma(Ssq, Z2, (2 * Z + Bsq) * BS2) * iDn;
   if (!(v2 < 1.0)) return false;
   const double iZ2 = iDn * ZB * ZB, iZ = iZ2 * Z;
   const double om = 1 - v2;
-  const double is = rsqrt(om), s = om * is;
+  const double is = RCP ? rsqrt64(om) : rsqrt(om), s = om * is;
   const double p = k * (Z * om - D * s);
   gv = Z + Bsq - p - 0.5 * Bsq * om - 0.5 * BS2 * iZ2 - D - tau;
   const double dv2 = (fma(2 * Ssq, Z, 2 * BS2) - v2 * (2 * Z * ZB * (2 * Z + Bsq))) * iDn;
@@ -59,6 +79,7 @@ __device__ __forceinline__ bool srmhd_g(double Z, double D, double tau, double B
 // The right end of the bracket is searched for only when a step needs it (an
 // unusable guess, v^2 >= 1, a step out of the bracket, a non-positive slope);
 // a Newton run that converges from a good guess never evaluates it.
+template <bool RCP>
 __device__ __forceinline__ bool newton_srmhd(double D, double tau, double BS2, double Bsq,
                                              double Ssq, double g, double& Z, double& vsq,
                                              int& iters) {
@@ -72,7 +93,7 @@ __device__ __forceinline__ bool newton_srmhd(double D, double tau, double BS2, d
     hi = fmax(g * (tau + D + Bsq), 1e-300);
     for (int q = 0; q < 64; ++q) {
       double gh, dh, vh;
-      if (srmhd_g(hi, D, tau, BS2, Bsq, Ssq, k, gh, dh, vh) && gh > 0) break;
+      if (srmhd_g<RCP>(hi, D, tau, BS2, Bsq, Ssq, k, gh, dh, vh) && gh > 0) break;
       hi *= 2;
     }
     have_hi = true;
@@ -85,7 +106,7 @@ __device__ __forceinline__ bool newton_srmhd(double D, double tau, double BS2, d
   for (int it = 0; it < 100; ++it) {
     ++iters;
     double Zn;
-    if (!srmhd_g(Zc, D, tau, BS2, Bsq, Ssq, k, gv, dg, v2)) {
+    if (!srmhd_g<RCP>(Zc, D, tau, BS2, Bsq, Ssq, k, gv, dg, v2)) {
       lo = Zc;  // v^2 >= 1: left of the root
       find_hi();
       Zn = lo > 0 ? sqrt(lo * hi) : 0.5 * hi;
@@ -101,7 +122,7 @@ __device__ __forceinline__ bool newton_srmhd(double D, double tau, double BS2, d
         hi = Zc;
         have_hi = true;
       }
-      Zn = Zc - gv / dg;
+      Zn = Zc - (RCP ? gv * rcp64(dg) : gv / dg);
       if (!(dg > 0) || !(Zn > lo && (!have_hi || Zn < hi))) {
         find_hi();
         Zn = (lo > 0 && hi > 4 * lo) ? sqrt(lo * hi) : 0.5 * (lo + hi);
@@ -109,7 +130,7 @@ __device__ __forceinline__ bool newton_srmhd(double D, double tau, double BS2, d
     }
     if (fabs(Zn - Zc) <= 1e-14 * Zn || (have_hi && hi - lo <= 1e-15 * hi)) {
       Zc = Zn;
-      if (!srmhd_g(Zc, D, tau, BS2, Bsq, Ssq, k, gv, dg, v2)) return false;
+      if (!srmhd_g<RCP>(Zc, D, tau, BS2, Bsq, Ssq, k, gv, dg, v2)) return false;
       Z = Zc;
       vsq = v2;
       break;
@@ -136,24 +157,31 @@ __device__ __forceinline__ void from_solution_fast(const double* c, const double
   a[11] = Bsq;
   a[12] = Ssq;
   const double om = 1 - sol[0];
-  const double W = rsqrt(om), iW = om * W;
+  const double W = rsqrt64(om), iW = om * W;
   a[1] = W;
   p[0] = c[0] * iW;
-  a[0] = sol[1] * iW / c[0];
-  const double ig = 1 / gamma;
+  a[0] = sol[1] * iW * rcp64(c[0]);
+  const double ig = rcp64(gamma);
   p[4] = (a[0] - 1) * p[0] * ((gamma - 1) * ig);
   a[2] = (a[0] - 1) * ig;
-  const double iq = 1 / (sol[1] * (Bsq + sol[1]));
+  const double iq = rcp64(sol[1] * (Bsq + sol[1]));
   p[1] = fma(c[5], BS, c[1] * sol[1]) * iq;
   p[2] = fma(c[6], BS, c[2] * sol[1]) * iq;
   p[3] = fma(c[7], BS, c[3] * sol[1]) * iq;
   a[9] = p[1] * p[1] + p[2] * p[2] + p[3] * p[3];
-  a[3] = sqrt((a[0] - 1) * (gamma - 1) / a[0]);
+  a[3] = sqrt((a[0] - 1) * (gamma - 1) * rcp64(a[0]));
   a[4] = W * (c[5] * p[1] + c[6] * p[2] + c[7] * p[3]);
   a[5] = fma(c[5], iW, a[4] * p[1]);
   a[6] = fma(c[6], iW, a[4] * p[2]);
   a[7] = fma(c[7], iW, a[4] * p[3]);
   a[8] = (Bsq + a[4] * a[4]) * om;
+}
+
+// Initial guess (v^2, rho h W^2) from the previous primitive state
+// (srmhd.cc:438-442).
+__device__ __forceinline__ void guess_from_prims_fast(const double* p, double h, double* sol) {
+  sol[0] = p[1] * p[1] + p[2] * p[2] + p[3] * p[3];
+  sol[1] = p[0] * h * rcp64(1 - sol[0]);
 }
 
 // Newton in Z for SRRMHD's residual (srrmhd.cc:512-537).
@@ -170,11 +198,11 @@ __device__ __forceinline__ bool newton_srrmhd(double Sb2, double D, double tauT,
       continue;
     }
     // one division and one reciprocal square root per step
-    const double iZ = 1 / Zc, Sz = Sb2 * iZ, q = Sz * iZ;
-    const double is = rsqrt(1 - q), s = (1 - q) * is;
+    const double iZ = rcp64(Zc), Sz = Sb2 * iZ, q = Sz * iZ;
+    const double is = rsqrt64(1 - q), s = (1 - q) * is;
     const double r = Zc - k * (Zc - Sz) + (k * s - 1) * D - tauT;
     const double dr = 1 - k * (1 + q) + k * D * q * iZ * is;
-    double Zn = Zc - r / dr;
+    double Zn = Zc - r * rcp64(dr);
     if (!(Zn > 0) || !isfinite(Zn)) Zn = 0.5 * Zc;
     if (fabs(Zn - Zc) <= 1e-13 * Zn) {
       if (!(Sb2 < Zn * Zn)) return false;
@@ -228,19 +256,19 @@ __device__ __forceinline__ void c2p_srmhd_newton_cell(const Grid& g, long long c
 #pragma unroll
   for (int v = 0; v < 4; ++v) pg[v] = prims_guess[v * N + cell];
   double prev[2];
-  srmhd::guess_from_prims(pg, aux_guess[cell], prev);
+  guess_from_prims_fast(pg, aux_guess[cell], prev);
   double Z = prev[1], vsq = prev[0];
   int it = 0;
   bool ok = false;
   if (guess_mode == 1 && zguess) {
     Z = zguess[cell];
-    ok = newton_srmhd(R.D, R.tau, BS2, R.Bsq, R.Ssq, g.gamma, Z, vsq, it);
+    ok = newton_srmhd<false>(R.D, R.tau, BS2, R.Bsq, R.Ssq, g.gamma, Z, vsq, it);
     if (!ok) {
       tl.fb_prev += 1;
       Z = prev[1];
     }
   }
-  if (!ok) ok = newton_srmhd(R.D, R.tau, BS2, R.Bsq, R.Ssq, g.gamma, Z, vsq, it);
+  if (!ok) ok = newton_srmhd<false>(R.D, R.tau, BS2, R.Bsq, R.Ssq, g.gamma, Z, vsq, it);
   double x[2] = {vsq, Z};
   if (!ok) {
     tl.fb_hybrd += 1;
@@ -295,6 +323,10 @@ __device__ __forceinline__ void tally_flush(NewtonTally tl, bool active, long lo
 // 512x1024 stages 5-15%.  With the Powell-hybrid fallback out of line the
 // SRMHD Newton kernels spill 80 bytes instead of 700 (0.083 -> 0.076 ms).
 constexpr int kNewtonMinBlocks = 8;     // 128 threads x 8 CTAs -> 64 registers
+// The SRRMHD recovery and the implicit stages, whose straight-line reciprocals
+// want more: 80 registers (SSP2 512x1024 step 0.424 ms; 0.429 at 64, 0.458
+// with the library's division and rsqrt at 64).
+constexpr int kSrrmhdMinBlocks = 6;
 
 template <bool LEAN>
 __global__ void __launch_bounds__(128, kNewtonMinBlocks)
@@ -357,15 +389,15 @@ __device__ __forceinline__ void c2p_srrmhd_newton_cell(const Grid& g, long long 
   // srrmhd.cc:283-301 with reciprocals: W = 1/sqrt(1 - v^2), rho = D/W,
   // h = Z/(rho W^2) = Z/(D W), c_s^2 = e gamma (gamma - 1)/h = (h - 1)(gamma - 1)/h
   a[10] = Z;
-  const double iZ = 1 / Z;
+  const double iZ = rcp64(Z);
   a[9] = a[15] * iZ * iZ;
   const double om = 1 - a[9];
-  a[1] = rsqrt(om);
+  a[1] = rsqrt64(om);
   const double iW = om * a[1];
   p[0] = c[0] * iW;
-  a[0] = Z * iW / c[0];
-  a[2] = (a[0] - 1) / gm;
-  a[3] = sqrt((a[0] - 1) * (gm - 1) / a[0]);
+  a[0] = Z * iW * rcp64(c[0]);
+  a[2] = (a[0] - 1) * rcp64(gm);
+  a[3] = sqrt((a[0] - 1) * (gm - 1) * rcp64(a[0]));
   p[4] = p[0] * a[2] * (gm - 1);
   p[1] = a[12] * iZ;
   p[2] = a[13] * iZ;
@@ -425,10 +457,10 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int v = 0; v < 4; ++v) pg[v] = prims_guess[v * N + cell];
       double prev[2];
-      srmhd::guess_from_prims(pg, aux_guess[cell], prev);
+      guess_from_prims_fast(pg, aux_guess[cell], prev);
       double Z = prev[1], vsq = prev[0];
       int it = 0;
-      bool ok = newton_srmhd(R.D, R.tau, BS2, R.Bsq, R.Ssq, g.gamma, Z, vsq, it);
+      bool ok = newton_srmhd<false>(R.D, R.tau, BS2, R.Bsq, R.Ssq, g.gamma, Z, vsq, it);
       double x[2] = {vsq, Z};
       if (!ok) {
         tl.fb_hybrd += 1;
@@ -470,7 +502,7 @@ __global__ void __launch_bounds__(128)
 }
 
 template <bool LEAN>
-__global__ void __launch_bounds__(128, kNewtonMinBlocks)
+__global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     k_c2p_newton_srrmhd(Grid g, const double* __restrict__ cons, const double* aux_guess,
                         double* prims, double* aux, C2PWork w, const double* zseed, long long t0,
                         long long t_end) {
@@ -485,11 +517,17 @@ __global__ void __launch_bounds__(128, kNewtonMinBlocks)
   tally_flush(tl, t < t_end, w.counters);
 }
 
-// Batched SRMHD primitive recovery for independent cells.
-__global__ void __launch_bounds__(128)
-    k_c2p_batch_srmhd(long long n, double gamma, int method, int guess,
-                      const double* __restrict__ cons, double* prims, double* aux,
-                      const double* __restrict__ zguess, long long* counters) {
+// Batched SRMHD primitive recovery for independent cells: METHOD 0 the
+// reference's Powell hybrid, 1 Newton with the fallbacks of the grid
+// recovery.  Each method has its kernel, so that Newton's registers (80, 6
+// CTAs on an SM) and code are not the hybrid's (156 for both).  Bound by FP64
+// latency, then by memory (35 planes of 8 bytes): 2^22 cells from a
+// previous-step guess 0.47 -> 0.34 ms, 2.5 -> 3.5 TB/s.
+template <int METHOD>
+__global__ void __launch_bounds__(128, METHOD == 1 ? 6 : 5)
+    k_c2p_batch_srmhd(long long n, double gamma, int guess, const double* __restrict__ cons,
+                      double* prims, double* aux, const double* __restrict__ zguess,
+                      long long* counters) {
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long its = 0, bad = 0, fb = 0;
   if (q < n) {
@@ -504,49 +542,47 @@ __global__ void __launch_bounds__(128)
       for (int v = 0; v < 4; ++v) pg[v] = prims[v * n + q];
       srmhd::guess_from_prims(pg, aux[q], prev);
     }
-    double x0[2];
+    double x[2];
     if (guess == 1) {
-      x0[0] = zguess[n + q];
-      x0[1] = zguess[q];
+      x[0] = zguess[n + q];
+      x[1] = zguess[q];
     } else if (guess == 2) {
       const double E = R.tau + R.D;
-      x0[1] = fmax(E, sqrt(R.Ssq) * 1.0000001);
-      x0[0] = fmin(R.Ssq / (x0[1] * x0[1]), 0.999999);
+      x[1] = fmax(E, sqrt(R.Ssq) * 1.0000001);
+      x[0] = fmin(R.Ssq / (x[1] * x[1]), 0.999999);
     } else {
-      x0[0] = prev[0];
-      x0[1] = prev[1];
+      x[0] = prev[0];
+      x[1] = prev[1];
     }
-    double x[2] = {x0[0], x0[1]}, fv[2];
+    double p[8], a[13];
     int it = 0;
     bool ok = false;
-    if (method == 1) {
-      double Z = x0[1], vsq = x0[0];
-      ok = newton_srmhd(R.D, R.tau, R.BS * R.BS, R.Bsq, R.Ssq, gamma, Z, vsq, it);
+    if constexpr (METHOD == 1) {
+      const double BS2 = R.BS * R.BS;
+      ok = newton_srmhd<true>(R.D, R.tau, BS2, R.Bsq, R.Ssq, gamma, x[1], x[0], it);
       if (!ok && guess != 0) {
         fb = 1;
-        Z = prev[1];
-        ok = newton_srmhd(R.D, R.tau, R.BS * R.BS, R.Bsq, R.Ssq, gamma, Z, vsq, it);
-      }
-      if (ok) {
-        x[0] = vsq;
-        x[1] = Z;
-      } else {
-        fb = 1;
-        x[0] = prev[0];
         x[1] = prev[1];
-        HybrdResult r = Hybrd<2>::solve(R, x, fv, 1.49011612e-7);
+        ok = newton_srmhd<true>(R.D, R.tau, BS2, R.Bsq, R.Ssq, gamma, x[1], x[0], it);
+      }
+      if (!ok) {
+        fb = 1;
+        const HybrdOut r = hybrd2_fallback(R, prev[0], prev[1]);
+        x[0] = r.x0;
+        x[1] = r.x1;
         it += r.nfev;
         ok = r.info == 1;
       }
+      from_solution_fast(c, x, gamma, R.BS, R.Bsq, R.Ssq, p, a);
     } else {
-      HybrdResult r = Hybrd<2>::solve(R, x, fv, 1.49011612e-7);
+      double fv[2];
+      const HybrdResult r = Hybrd<2>::solve(R, x, fv, 1.49011612e-7);
       it = r.nfev;
       ok = r.info == 1;
+      srmhd::from_solution(c, x, gamma, R.BS, R.Bsq, R.Ssq, p, a);
     }
     bad = ok ? 0 : 1;
     its = it;
-    double p[8], a[13];
-    srmhd::from_solution(c, x, gamma, R.BS, R.Bsq, R.Ssq, p, a);
 #pragma unroll
     for (int v = 0; v < 8; ++v) prims[v * n + q] = p[v];
 #pragma unroll
@@ -591,9 +627,9 @@ __device__ __forceinline__ bool srrmhd_prims_newton(const double* x, double g, d
   const double Esq = x[8] * x[8] + x[9] * x[9] + x[10] * x[10];
   const double tauB = x[4] - 0.5 * (Bsq + Esq);
   if (!newton_srrmhd(Sbsq, x[0], tauB, g, Z, its)) return false;
-  const double iZ = 1 / Z;
+  const double iZ = rcp64(Z);
   const double vsq = Sbsq * iZ * iZ;
-  W = rsqrt(1 - vsq);
+  W = rsqrt64(1 - vsq);
   v[0] = Sb0 * iZ;
   v[1] = Sb1 * iZ;
   v[2] = Sb2 * iZ;
@@ -635,8 +671,9 @@ __device__ __forceinline__ bool imex_fast_form(const Grid& g, long long cell,
   }
   // D has no source: x[0] = c[0] throughout, so the conductivity is fixed per cell
   const double a = FORM <= 3 ? dt * kGam : 0.5 * dt, cp2 = g.cp * g.cp, sg = sigma_of(g, c[0]);
-  x[12] = c[12] / (1 + a / cp2);
-  x[11] = (c[11] + a * c[13]) / (1 + a / cp2);
+  const double ip = rcp64(1 + a * rcp64(cp2));
+  x[12] = c[12] * ip;
+  x[11] = (c[11] + a * c[13]) * ip;
   // the inner recovery's Z: the network's guess for the stage's first
   // iterate when given (the previous state's Z is its fallback), else that Z
   double Z = zseed ? zseed[cell] : aux_guess[10 * N + cell];
@@ -662,8 +699,8 @@ __device__ __forceinline__ bool imex_fast_form(const Grid& g, long long cell,
     const double beta = a * Ws, alpha = 1 + beta;
     const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
     const double vR = v[0] * R[0] + v[1] * R[1] + v[2] * R[2];
-    const double iA = 1 / alpha;
-    const double f = beta * vR * iA / (alpha - beta * vv);
+    const double iA = rcp64(alpha);
+    const double f = beta * vR * iA * rcp64(alpha - beta * vv);
     double dE[3];
     dE[0] = -(R[0] * iA + f * v[0]);
     dE[1] = -(R[1] * iA + f * v[1]);
@@ -719,7 +756,7 @@ __global__ void __launch_bounds__(128)
 
 // SSP3 / SSP2322 stages in the mixed form; failures queued for the exact solve.
 template <int FORM>
-__global__ void __launch_bounds__(128, kNewtonMinBlocks)
+__global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     k_imex_fast_form(Grid g, const double* __restrict__ cons, const double* zaux,
                      const double* __restrict__ flux1, const double* __restrict__ flux2,
                      const double* __restrict__ source1, const double* __restrict__ source2,
@@ -747,7 +784,7 @@ __global__ void __launch_bounds__(128, kNewtonMinBlocks)
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(128, kNewtonMinBlocks)
+__global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     k_imex_fast(Grid g, const double* __restrict__ cons, const double* __restrict__ aux_guess,
                 const double* __restrict__ u1, const double* __restrict__ flux1,
                 const double* __restrict__ source1, double* __restrict__ out, double dt,
@@ -796,7 +833,7 @@ __global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, float, ORDER, TI
 // One model's members per launch (the work list holds one model's cells), so
 // each instantiation carries one recovery method's registers.
 template <int MODEL, bool LEAN>
-__global__ void __launch_bounds__(128, kNewtonMinBlocks)
+__global__ void __launch_bounds__(128, MODEL == MODEL_SRMHD ? kNewtonMinBlocks : kSrrmhdMinBlocks)
     k_ens_c2p_newton(const Member* __restrict__ mem, const Item* __restrict__ items, int n_items,
                      int guess_mode, int ic, int ipg, int iag, int ip, int ia) {
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
@@ -844,7 +881,7 @@ __global__ void __launch_bounds__(128)
 }
 
 template <int STAGE>
-__global__ void __launch_bounds__(128, kNewtonMinBlocks)
+__global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     k_ens_imex_fast(const Member* __restrict__ mem, const Item* __restrict__ items, int n_items,
                     int guess_mode) {
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
@@ -1012,8 +1049,11 @@ cudaError_t launch_fvs2d_fp32(const Grid& g, int model, int order, const double*
 cudaError_t launch_c2p_batch(long long n, double gamma, int method, int guess,
                              const double* cons, double* prims, double* aux,
                              const double* zguess, long long* counters, cudaStream_t st) {
-  k_c2p_batch_srmhd<<<(int)((n + 127) / 128), 128, 0, st>>>(n, gamma, method, guess, cons, prims,
-                                                              aux, zguess, counters);
+  const int b = (int)((n + 127) / 128);
+  if (method == 1)
+    k_c2p_batch_srmhd<1><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
+  else
+    k_c2p_batch_srmhd<0><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
   return cudaGetLastError();
 }
 

@@ -1,0 +1,50 @@
+"""Batched SRMHD recovery at the edges of its launches (blocks of 128 cells)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from method_b200 import initial
+
+pytestmark = pytest.mark.gpu
+
+G = 4.0 / 3.0
+
+
+def conserved(p):
+    rho, v, pr, B = p[0], p[1:4], p[4], p[5:8]
+    W = 1 / np.sqrt(1 - (v * v).sum(0))
+    h = 1 + pr / rho * (G / (G - 1))
+    b0 = W * (v * B).sum(0)
+    b = B / W + b0 * v
+    bsq = ((B * B).sum(0) + b0 * b0) / (W * W)
+    q = (rho * h + bsq) * W * W
+    tau = q - (pr + bsq / 2) - b0 * b0 - rho * W
+    return np.concatenate([[rho * W], q * v - b0 * b, [tau], B, [0 * rho]]), h
+
+
+@pytest.mark.parametrize("n", [1, 31, 128, 129, 1000])
+@pytest.mark.parametrize("method,guess", [(0, 0), (1, 0), (1, 2)])
+def test_batch_recovers_generating_states(n, method, guess):
+    """Newton from a previous state 1% off and from a cold start, the Powell
+    hybrid from the state itself.  The inversion magnifies the rounding of the
+    conserved state by up to W^4 (1 + b^2 / rho) of a few 1e6: 1e-8."""
+    import torch
+
+    from method_b200 import _lib
+    L = _lib.load()
+    p = initial.random_c2p_states(n, seed=n)
+    cons, h = conserved(p)
+    pg, ag = np.zeros((8, n)), np.zeros((13, n))
+    off = 0.0 if method == 0 else 0.01
+    pg[0], pg[1:4], ag[0] = p[0] * (1 + off), p[1:4] * (1 - off), h * (1 + off)
+    dc, dp, da = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (cons, pg, ag))
+    st = _lib.C2PBatchStats()
+    rc = L.mth_c2p_batch(G, n, dc.data_ptr(), dp.data_ptr(), da.data_ptr(), method, guess, None,
+                         None, None, C.byref(st))
+    assert rc == 0 and st.cells == n and st.unconverged == 0
+    got, aux = dp.cpu().numpy(), da.cpu().numpy()
+    assert np.max(np.abs(got[0] - p[0]) / p[0]) < 1e-8
+    assert np.max(np.abs(got[1:4] - p[1:4])) < 1e-8
+    assert np.array_equal(got[5:8], p[5:8])
+    assert np.max(np.abs(aux[0] - h) / h) < 1e-7  # h - 1 is down to 4e-3 of h
