@@ -404,12 +404,13 @@ cudaError_t enqueue_ssp2_part(mth_handle* h, double dt, int part) {
       return e;
     return c2p(h, h->cons, h->prims, h->aux, h->prims, h->aux);
   }
-  if ((e = timed(h, "source", 31, [&] {
+  // the mixed stage 2 forms S(U1) itself, except with the guess network
+  if ((!fast || mlp_work(h)) && (e = timed(h, "source", 31, [&] {
          return launch_source(h->g, h->cfg.model, h->u1, h->aux, h->src1, h->st);
        })))
     return e;
   if ((e = flux_stage(h, h->u1, h->prims, h->aux, nullptr, h->flux1, dt, STAGE_FNET))) return e;
-  if ((e = timed(h, fast ? "imex_newton_stage2" : "imex_hybrd_stage2", 71, [&] {
+  if ((e = timed(h, fast ? "imex_newton_stage2" : "imex_hybrd_stage2", fast ? 54 : 71, [&] {
          return fast ? launch_imex_fast(h->g, 2, h->cons, h->aux, h->u1, h->flux1, h->src1,
                                         h->u2, dt, imex_work(h), h->st, mlp_work(h))
                      : launch_imex_stage(h->g, 2, h->cons, h->aux, h->u1, h->flux1, h->src1,

@@ -262,7 +262,8 @@ cudaError_t srrmhd_ssp2(mth_ensemble* e, cudaStream_t s) {
       return r;
     if ((r = c2p_phase(e, s, md, u, EA_PRIMS, EA_AUX, EA_PRIMS, EA_AUX, true))) return r;
     if (stage == 2) break;
-    if ((r = phase(e, s, "source", [&] {
+    // without the network stage 2 forms S(U1) itself
+    if (gm && (r = phase(e, s, "source", [&] {
            return ens_source(e->d_mem, it, n, u, EA_AUX, EA_S1, grid, s);
          })))
       return r;

@@ -174,7 +174,8 @@ __device__ __forceinline__ void stage_update(const Grid& g, const double* __rest
 #pragma unroll
     for (int v = 0; v < NC; ++v) {
       const long long o = (long long)v * g.Ntot + cell;
-      out[o] = u0[o] + -0.5 * dt * (tail.flux1[o] + (double)acc[v] - tail.source1[o] - s2[v]);
+      const double s1 = M::sourced(v) ? tail.source1[o] : 0.0;
+      out[o] = u0[o] + -0.5 * dt * (tail.flux1[o] + (double)acc[v] - s1 - s2[v]);
     }
     return;
   }
@@ -206,7 +207,7 @@ __device__ __forceinline__ void prefetch_tail(const Grid& g, const double* u0, i
     asm volatile("prefetch.global.L2 [%0];" ::"l"(u0 + o));
     if (mode == STAGE_SSP2_FINAL) {
       asm volatile("prefetch.global.L2 [%0];" ::"l"(tail.flux1 + o));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(tail.source1 + o));
+      if (M::sourced(v)) asm volatile("prefetch.global.L2 [%0];" ::"l"(tail.source1 + o));
     }
   }
 }

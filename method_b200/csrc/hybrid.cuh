@@ -82,6 +82,7 @@ struct HYBRID {
                                                 int dir, R* f) {
     hybrid_flux<R>(g, c, p, a, dir, f);
   }
+  __host__ __device__ static constexpr bool sourced(int) { return true; }
   // The SSP2 closing stage does not run with this model (RK2 and RKSplit2
   // only); the tile's stage epilogue still names a cell source.
   __device__ __forceinline__ static void cell_source(const double* __restrict__,

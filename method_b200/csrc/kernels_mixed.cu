@@ -646,24 +646,45 @@ __device__ __forceinline__ bool srrmhd_prims_newton(const double* x, double g, d
 // forms; E is Newton-iterated with the stiff Jacobian inverted by
 // Sherman-Morrison (v frozen per step).  The final Z goes to zout[10] when
 // zout is given (the seed of the stage's recovery).
+// FORM 2 with u1 given: aux_guess is the recovered aux of U1 and the stage
+// forms S(U1) itself (rows 8-12, srrmhd.cc:194-206; the others are zero) from
+// J and u1, into source1 for the closing combination; no separate pass writes
+// and reads 14 planes for it (SSP2 512x1024 step
+// 0.423 -> 0.398 ms).
 template <int FORM>
 __device__ __forceinline__ bool imex_fast_form(const Grid& g, long long cell,
                                                const double* __restrict__ cons,
                                                const double* __restrict__ aux_guess,
                                                const double* __restrict__ flux1,
                                                const double* __restrict__ flux2,
-                                               const double* __restrict__ source1,
+                                               double* source1,
                                                const double* __restrict__ source2,
                                                double* __restrict__ out, double* zout, double dt,
-                                               int& its, const double* zseed = nullptr) {
+                                               int& its, const double* zseed = nullptr,
+                                               const double* __restrict__ u1 = nullptr) {
   const long long N = g.Ntot;
-  double c[14], x[14];
+  double c[14], x[14], s1[14];
+  if (FORM == 2) {
+#pragma unroll
+    for (int v = 0; v < 14; ++v)
+      s1[v] = u1 || !SRRMHD::sourced(v) ? 0.0 : source1[v * N + cell];
+    if (u1) {
+      double a[17];
+#pragma unroll
+      for (int v = 4; v < 7; ++v) a[v] = aux_guess[v * N + cell];
+#pragma unroll
+      for (int v = 11; v < 14; ++v) x[v] = u1[v * N + cell];
+      srrmhd::source(x, a, g.cp, s1);
+#pragma unroll
+      for (int v = 8; v < 13; ++v) source1[v * N + cell] = s1[v];
+    }
+  }
 #pragma unroll
   for (int v = 0; v < 14; ++v) {
     const long long o = v * N + cell;
     const double u = cons[o];
     if (FORM == 1 || FORM == 4) c[v] = u;
-    else if (FORM == 2) c[v] = u - dt * (flux1[o] - kOm2Gam * source1[o]);
+    else if (FORM == 2) c[v] = u - dt * (flux1[o] - kOm2Gam * s1[v]);
     else if (FORM == 3) c[v] = u - dt * (flux1[o] + flux2[o]) / 4.0 + dt * kHmGam * source1[o];
     else if (FORM == 5) c[v] = u - 0.5 * dt * source1[o];
     else c[v] = u - dt * (flux2[o] - 0.5 * source2[o]);
@@ -726,12 +747,12 @@ template <int STAGE>
 __device__ __forceinline__ bool imex_fast_cell(const Grid& g, long long cell,
                                                const double* __restrict__ cons,
                                                const double* __restrict__ aux_guess,
-                                               const double* __restrict__ flux1,
-                                               const double* __restrict__ source1,
+                                               const double* __restrict__ flux1, double* source1,
                                                double* __restrict__ out, double dt, int& its,
-                                               const double* zseed = nullptr) {
+                                               const double* zseed = nullptr,
+                                               const double* __restrict__ u1 = nullptr) {
   return imex_fast_form<STAGE>(g, cell, cons, aux_guess, flux1, nullptr, source1, nullptr, out,
-                               nullptr, dt, its, zseed);
+                               nullptr, dt, its, zseed, u1);
 }
 
 // The first iterate of SSP2 implicit stage STAGE (the stage's explicit part
@@ -759,7 +780,7 @@ template <int FORM>
 __global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     k_imex_fast_form(Grid g, const double* __restrict__ cons, const double* zaux,
                      const double* __restrict__ flux1, const double* __restrict__ flux2,
-                     const double* __restrict__ source1, const double* __restrict__ source2,
+                     double* source1, const double* __restrict__ source2,
                      double* __restrict__ out, double* zout, double dt, C2PWork w) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long its_total = 0;
@@ -787,9 +808,8 @@ template <int STAGE>
 __global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     k_imex_fast(Grid g, const double* __restrict__ cons, const double* __restrict__ aux_guess,
                 const double* __restrict__ u1, const double* __restrict__ flux1,
-                const double* __restrict__ source1, double* __restrict__ out, double dt,
-                C2PWork w, const double* zseed) {
-  (void)u1;
+                double* source1, double* __restrict__ out, double dt, C2PWork w,
+                const double* zseed) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long its_total = 0;
   if (t < n_interior(g)) {
@@ -797,8 +817,8 @@ __global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
     interior_ijk(g, t, i, j, k);
     const long long cell = cell_id(g, i, j, k);
     int its = 0;
-    if (!imex_fast_cell<STAGE>(g, cell, cons, aux_guess, flux1, source1, out, dt, its,
-                               zseed)) {
+    if (!imex_fast_cell<STAGE>(g, cell, cons, aux_guess, flux1, source1, out, dt, its, zseed,
+                               u1)) {
       const int slot = atomicAdd(w.fail_count, 1);
       w.fail_list[slot] = (int)cell;
     }
@@ -898,7 +918,8 @@ __global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
       const long long cell = cell_id(g, i, j, k);
       const bool ok = imex_fast_cell<STAGE>(g, cell, d.a[EA_CONS], d.a[EA_AUX], d.a[EA_F1],
                                             d.a[EA_S1], d.a[STAGE == 1 ? EA_U1 : EA_U2], d.dt,
-                                            its, guess_mode ? d.a[EA_ZG] : nullptr);
+                                            its, guess_mode ? d.a[EA_ZG] : nullptr,
+                                            guess_mode ? nullptr : d.a[EA_U1]);
       its_total = its;
       if (!ok) {  // queued for the reference solve (ens_imex_queued)
         const int slot = atomicAdd(d.fail_count, 1);
@@ -1110,12 +1131,14 @@ cudaError_t launch_c2p_hybrid_mixed(const Grid& g, const double* cons, const dou
 
 cudaError_t launch_imex_fast(const Grid& g, int stage, const double* cons,
                              const double* aux_guess, const double* u1, const double* flux1,
-                             const double* source1, double* out, double dt, C2PWork w,
+                             double* source1, double* out, double dt, C2PWork w,
                              cudaStream_t st, const MixedWork* mw) {
   const long long nI = (long long)(g.ie - g.is) * (g.je - g.js) * (g.ke - g.ks);
   const int blocks = (int)((nI + 127) / 128);
   const double* zseed = nullptr;
+  const double* from_u1 = u1;
   if (mw && mw->has_mlp) {
+    from_u1 = nullptr;  // source1 is given: the network's input reads it too
     // the network's Z for the stage's first iterate, its explicit part: U^n
     // itself for stage 1; for stage 2 staged in `out` (which the stage then
     // overwrites)
@@ -1128,11 +1151,11 @@ cudaError_t launch_imex_fast(const Grid& g, int stage, const double* cons,
     zseed = mw->zguess;
   }
   if (stage == 1)
-    k_imex_fast<1><<<blocks, 128, 0, st>>>(g, cons, aux_guess, u1, flux1, source1, out, dt, w,
-                                           zseed);
+    k_imex_fast<1><<<blocks, 128, 0, st>>>(g, cons, aux_guess, nullptr, flux1, source1, out, dt,
+                                           w, zseed);
   else
-    k_imex_fast<2><<<blocks, 128, 0, st>>>(g, cons, aux_guess, u1, flux1, source1, out, dt, w,
-                                           zseed);
+    k_imex_fast<2><<<blocks, 128, 0, st>>>(g, cons, aux_guess, from_u1, flux1, source1, out, dt,
+                                           w, zseed);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // cells the fast solve could not converge: the reference stage solve
@@ -1142,7 +1165,7 @@ cudaError_t launch_imex_fast(const Grid& g, int stage, const double* cons,
 cudaError_t launch_imex_fast_form(const Grid& g, int form, const double* cons,
                                   const double* zaux, const double* u1, const double* u2,
                                   const double* flux1, const double* flux2,
-                                  const double* source1, const double* source2, double* out,
+                                  double* source1, const double* source2, double* out,
                                   double* zout, double dt, C2PWork w, cudaStream_t st) {
   const int blocks = (int)((n_interior_host(g) + 127) / 128);
 #define FAST(F)                                                                          \

@@ -37,13 +37,13 @@ cudaError_t launch_zguess(const Grid& g, long long n_cells, bool batch, const do
 cudaError_t launch_imex_fast_form(const Grid& g, int form, const double* cons,
                                   const double* zaux, const double* u1, const double* u2,
                                   const double* flux1, const double* flux2,
-                                  const double* source1, const double* source2, double* out,
+                                  double* source1, const double* source2, double* out,
                                   double* zout, double dt, C2PWork w, cudaStream_t st);
 // mw (may be null): with a guess network installed, the inner recoveries
 // start from its Z for the stage's first iterate.
 cudaError_t launch_imex_fast(const Grid& g, int stage, const double* cons,
                              const double* aux_guess, const double* u1, const double* flux1,
-                             const double* source1, double* out, double dt, C2PWork w,
+                             double* source1, double* out, double dt, C2PWork w,
                              cudaStream_t st, const MixedWork* mw = nullptr);
 
 // Batched primitive recovery of independent cells (variable-major, stride n).

@@ -228,6 +228,8 @@ struct SRMHD {
                                                 int dir, R* f) {
     srmhd::flux<R>(c, p, a, dir, f);
   }
+  // The variables whose source is not identically zero: phi.
+  __host__ __device__ static constexpr bool sourced(int v) { return v == 8; }
   // Model::sourceTerm of one cell in FP64 (srmhd.cc:215-250): S_phi = -phi/cp^2.
   __device__ __forceinline__ static void cell_source(const double* __restrict__ cons,
                                                      const double*, long long N, long long cell,

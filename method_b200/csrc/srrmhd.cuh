@@ -278,6 +278,8 @@ struct SRRMHD {
                                                 int dir, R* f) {
     srrmhd::flux<R>(c, p, a, dir, f);
   }
+  // The variables whose source is not identically zero: E, psi, phi.
+  __host__ __device__ static constexpr bool sourced(int v) { return v >= 8 && v <= 12; }
   // Model::sourceTerm of one cell in FP64 (srrmhd.cc:194-206): reads cons
   // 11-13 and aux 4-6 only.
   __device__ __forceinline__ static void cell_source(const double* __restrict__ cons,
