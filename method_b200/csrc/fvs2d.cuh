@@ -161,18 +161,18 @@ struct FaceScale<float> {
 // corrector 1/2 (U^n + U^1 - dt fnet), or SSP2's final combination
 // cons += -0.5 dt (flux1 + flux2 - source1 - source2) in the reference's
 // order (SSP2.cc:155-166) with flux2 = fnet and source2 = S(stage state).
-template <class M, typename R>
+// Variables [V0, V0 + NV).
+template <class M, typename R, int V0 = 0, int NV = M::NC>
 __device__ __forceinline__ void stage_update(const Grid& g, const double* __restrict__ cons,
                                              const double* __restrict__ aux, const double* u0,
                                              double* out, double dt, int mode,
                                              const StageTail& tail, long long cell,
                                              const R* acc) {
-  constexpr int NC = M::NC;
   if (mode == STAGE_SSP2_FINAL) {
-    double s2[NC];
+    double s2[M::NC];
     M::cell_source(cons, aux, g.Ntot, cell, tail.cp, s2);
 #pragma unroll
-    for (int v = 0; v < NC; ++v) {
+    for (int v = V0; v < V0 + NV; ++v) {
       const long long o = (long long)v * g.Ntot + cell;
       const double s1 = M::sourced(v) ? tail.source1[o] : 0.0;
       out[o] = u0[o] + -0.5 * dt * (tail.flux1[o] + (double)acc[v] - s1 - s2[v]);
@@ -180,7 +180,7 @@ __device__ __forceinline__ void stage_update(const Grid& g, const double* __rest
     return;
   }
 #pragma unroll
-  for (int v = 0; v < NC; ++v) {
+  for (int v = V0; v < V0 + NV; ++v) {
     const long long o = (long long)v * g.Ntot + cell;
     const double fn = (double)acc[v];
     if (mode == STAGE_FNET) {
@@ -197,12 +197,12 @@ __device__ __forceinline__ void stage_update(const Grid& g, const double* __rest
 // the RK2 corrector; U^n, flux1 and source1 of SSP2's final combination),
 // requested into L2 when the tile starts so that their latency overlaps the
 // flux phases (OT 1024^2 corrector tile: 0.154 -> 0.151 ms average launch).
-template <class M>
+template <class M, int V0 = 0, int NV = M::NC>
 __device__ __forceinline__ void prefetch_tail(const Grid& g, const double* u0, int mode,
                                               const StageTail& tail, long long cell) {
   if (mode != STAGE_RK2_CORR && mode != STAGE_SSP2_FINAL) return;
 #pragma unroll
-  for (int v = 0; v < M::NC; ++v) {
+  for (int v = V0; v < V0 + NV; ++v) {
     const long long o = (long long)v * g.Ntot + cell;
     asm volatile("prefetch.global.L2 [%0];" ::"l"(u0 + o));
     if (mode == STAGE_SSP2_FINAL) {

@@ -43,9 +43,9 @@ __device__ __forceinline__ void split_group(const Grid& g, const double* __restr
 }
 
 // Pass Q: the x and y flux differences of variables [Q G, Q G + NV) into
-// acc.  Ends with a barrier, so the next pass may reuse shared memory.
-template <class M, int ORDER, int TI, int G, int Q>
-__device__ __forceinline__ void group_pass(const Grid& g, const double* __restrict__ cons,
+// acc, PAIR as for weno_face.
+template <class M, int ORDER, int TI, int G, int Q, bool PAIR>
+__device__ __forceinline__ void group_one(const Grid& g, const double* __restrict__ cons,
                                            const double* __restrict__ prims,
                                            const double* __restrict__ aux, int i0, int j0,
                                            double* acc, unsigned char* smem_raw) {
@@ -69,7 +69,7 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
   const Divisor over_dx(g.dx);
   for (int e = tid, v = 0, fi = ty; e < NV * S::FX; e += NT) {
     sr[e] = over_dx(
-        weno_face<ORDER, double, false>(sp + v * S::RX + lane, sm + v * S::RX + lane, TJ, fi));
+        weno_face<ORDER, double, PAIR>(sp + v * S::RX + lane, sm + v * S::RX + lane, TJ, fi));
     fi += TI;
     if (fi > TI) {
       fi -= TI + 1;
@@ -97,7 +97,7 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
     int v = 0, r = tid / (TJ + 1), fj = tid % (TJ + 1);
     for (int e = tid; e < NV * S::FY; e += NT) {
       sr[e] = over_dy(
-          weno_face<ORDER, double, false>(sp + v * S::RY + r * WY, sm + v * S::RY + r * WY, 1, fj));
+          weno_face<ORDER, double, PAIR>(sp + v * S::RY + r * WY, sm + v * S::RY + r * WY, 1, fj));
       fj += FS;
       r += RS;
       if (fj > TJ) {
@@ -115,9 +115,19 @@ __device__ __forceinline__ void group_pass(const Grid& g, const double* __restri
   for (int v = 0; v < NV; ++v)
     acc[V0 + v] = acc[V0 + v] + (sr[v * S::FY + ty * (TJ + 1) + lane + 1] -
                                  sr[v * S::FY + ty * (TJ + 1) + lane]);
-  __syncthreads();
-  if constexpr (Q + 1 < Fvs2dGroupSmem<M, ORDER, TI, G>::NG)
+}
+
+// Passes Q, Q + 1, ...; a barrier between two, as they share the memory.
+template <class M, int ORDER, int TI, int G, int Q>
+__device__ __forceinline__ void group_pass(const Grid& g, const double* __restrict__ cons,
+                                           const double* __restrict__ prims,
+                                           const double* __restrict__ aux, int i0, int j0,
+                                           double* acc, unsigned char* smem_raw) {
+  group_one<M, ORDER, TI, G, Q, false>(g, cons, prims, aux, i0, j0, acc, smem_raw);
+  if constexpr (Q + 1 < Fvs2dGroupSmem<M, ORDER, TI, G>::NG) {
+    __syncthreads();
     group_pass<M, ORDER, TI, G, Q + 1>(g, cons, prims, aux, i0, j0, acc, smem_raw);
+  }
 }
 
 template <class M, int ORDER, int TI, int G, int MINB>
@@ -133,6 +143,44 @@ __global__ void __launch_bounds__(32 * TI, MINB)
   group_pass<M, ORDER, TI, G, 0>(g, cons, prims, aux, i0, j0, acc, smem_raw);
   if (ci < g.ie && cj < g.je)
     stage_update<M, double>(g, cons, aux, u0, out, dt, mode, tail, cell_id(g, ci, cj, 0), acc);
+}
+
+// The same tile with one CTA per group of G variables (blockIdx.z), for
+// grids of too few tiles to fill the chip: a thread then has a G-th of the
+// dependent face evaluations, which is what such a launch waits for, and the
+// groups run on SMs that would be idle.  Each CTA updates its own variables;
+// no stage mode writes what another CTA reads.
+template <class M, int ORDER, int TI, int G, int Q>
+__device__ __forceinline__ void group_cta(const Grid& g, const double* __restrict__ cons,
+                                          const double* __restrict__ prims,
+                                          const double* __restrict__ aux, const double* u0,
+                                          double* out, double dt, int mode, const StageTail& tail,
+                                          unsigned char* smem_raw) {
+  if constexpr (Q < Fvs2dGroupSmem<M, ORDER, TI, G>::NG) {
+    if (blockIdx.z != Q) {
+      group_cta<M, ORDER, TI, G, Q + 1>(g, cons, prims, aux, u0, out, dt, mode, tail, smem_raw);
+      return;
+    }
+    constexpr int V0 = Q * G, NV = M::NC - V0 < G ? M::NC - V0 : G;
+    const int i0 = g.is + blockIdx.y * TI, j0 = g.js + blockIdx.x * 32;
+    const int ci = i0 + threadIdx.y, cj = j0 + threadIdx.x;
+    const bool own = ci < g.ie && cj < g.je;
+    if (own) prefetch_tail<M, V0, NV>(g, u0, mode, tail, cell_id(g, ci, cj, 0));
+    double acc[M::NC];
+    group_one<M, ORDER, TI, G, Q, true>(g, cons, prims, aux, i0, j0, acc, smem_raw);
+    if (own)
+      stage_update<M, double, V0, NV>(g, cons, aux, u0, out, dt, mode, tail,
+                                      cell_id(g, ci, cj, 0), acc);
+  }
+}
+
+template <class M, int ORDER, int TI, int G>
+__global__ void __launch_bounds__(32 * TI)
+    k_fvs2d_group_ctas(Grid g, const double* __restrict__ cons, const double* __restrict__ prims,
+                       const double* __restrict__ aux, const double* u0, double* out, double dt,
+                       int mode, StageTail tail) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  group_cta<M, ORDER, TI, G, 0>(g, cons, prims, aux, u0, out, dt, mode, tail, smem_raw);
 }
 
 }  // namespace mth

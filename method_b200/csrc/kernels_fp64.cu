@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "ensemble.h"
@@ -579,11 +580,18 @@ __global__ void __launch_bounds__(128)
 // registers, a few spilled), WENO7 3, WENO9/11 2.  OT 1024^2 WENO5: two
 // passes of 5 + 4 variables 0.515 ms per launch, three of 3 0.549 ms (0.600
 // at 3 CTAs per SM), the one-pass tile 0.66 ms.
-// Grids of fewer than two tiles per SM keep the one-pass tile: there the
-// passes only lengthen each CTA (KH 64 x 128: 0.145 against 0.131 ms per
-// step).  Both forms give the same bits.
+// Grids of fewer than two tiles per SM run one CTA per tile and group of
+// variables: of one variable while that makes at most four CTAs per SM, else of
+// three (five for the Hybrid model, whose flux costs more to evaluate again
+// per group).  Plain RK2 steps with the tile's variables in one CTA, one per
+// CTA, three per CTA: KH 64 x 128 WENO3 (32 tiles) 65, 47, 50 us; OT 128 x 128
+// WENO5 (64) 87, 68, 71; 200 x 256 (200) 107, 98, 94; SRRMHD 200 x 256 96, 78, 63;
+// 256 x 288 (288) 86, 97, 86.  At two tiles per SM and above the grouped tile
+// is as fast with fewer loads.  All forms give the same bits.
 template <class M>
 constexpr int kFp64Group = 5;
+template <class M>
+constexpr int kFp64SmallGroup = std::is_same<M, HYBRID>::value ? 5 : 3;
 template <int ORDER>
 constexpr int kFp64Blocks = ORDER <= 5 ? 4 : ORDER <= 7 ? 3 : 2;
 
@@ -594,28 +602,40 @@ int device_sm_count() {
   return sms;
 }
 
+template <class M, int ORDER, int TI, int G>
+cudaError_t fvs2d_group_ctas(const Grid& g, const double* cons, const double* prims,
+                             const double* aux, const double* u0, double* out, double dt, int mode,
+                             StageTail tail, dim3 grid, cudaStream_t st) {
+  using S = Fvs2dGroupSmem<M, ORDER, TI, G>;
+  auto kern = k_fvs2d_group_ctas<M, ORDER, TI, G>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
+  if (e != cudaSuccess) return e;
+  grid.z = S::NG;
+  kern<<<grid, dim3(32, TI), S::bytes, st>>>(g, cons, prims, aux, u0, out, dt, mode, tail);
+  return cudaGetLastError();
+}
+
 template <class M, int ORDER, int TI>
 cudaError_t fvs2d_instance(const Grid& g, const double* cons, const double* prims,
                            const double* aux, const double* u0, double* out, double dt, int mode,
                            StageTail tail, cudaStream_t st) {
   dim3 grid((g.je - g.js + 31) / 32, (g.ie - g.is + TI - 1) / TI);
   dim3 block(32, TI);
-  if ((long long)grid.x * grid.y >= 2LL * device_sm_count()) {
+  const long long tiles = (long long)grid.x * grid.y, sms = device_sm_count();
+  if (tiles >= 2 * sms) {
     using S = Fvs2dGroupSmem<M, ORDER, TI, kFp64Group<M>>;
     auto kern = k_fvs2d_group<M, ORDER, TI, kFp64Group<M>, kFp64Blocks<ORDER>>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)S::bytes);
     if (e != cudaSuccess) return e;
     kern<<<grid, block, S::bytes, st>>>(g, cons, prims, aux, u0, out, dt, mode, tail);
-  } else {
-    using S = Fvs2dSmem<M, double, ORDER, TI>;
-    auto kern = k_fvs2d<M, double, ORDER, TI>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)S::bytes);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, block, S::bytes, st>>>(g, cons, prims, aux, u0, out, dt, mode, tail, 0);
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
+  if (tiles * M::NC <= 4LL * sms)
+    return fvs2d_group_ctas<M, ORDER, TI, 1>(g, cons, prims, aux, u0, out, dt, mode, tail, grid, st);
+  return fvs2d_group_ctas<M, ORDER, TI, kFp64SmallGroup<M>>(g, cons, prims, aux, u0, out, dt, mode,
+                                                            tail, grid, st);
 }
 
 // ---------------------------------------------------------------------------

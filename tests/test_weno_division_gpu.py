@@ -49,22 +49,27 @@ def test_flux_of_any_size_matches_oracle(weno, nx, ny, nz, scale):
 
 
 @pytest.mark.parametrize("weno", [3, 5])
-@pytest.mark.parametrize("nx,ny", [(8, 32), (7, 31), (9, 33), (17, 70), (100, 736)])
-@pytest.mark.parametrize("bcs", ["periodic", "outflow"])
-def test_fused_step_matches_oracle(weno, nx, ny, bcs):
-    """One RK2 step of a blast with constant regions, by the one-pass tile and,
-    at 100 x 736 (299 tiles), by the grouped one."""
+@pytest.mark.parametrize("nx,ny", [(8, 32), (7, 31), (9, 33), (17, 70), (100, 300), (100, 736)])
+@pytest.mark.parametrize("model,bcs", [("srmhd", "periodic"), ("srmhd", "outflow"),
+                                       ("srrmhd", "flow")])
+def test_fused_step_matches_oracle(weno, nx, ny, model, bcs):
+    """One RK2 step of a blast with constant regions, by a CTA per variable, by
+    CTAs of three (100 x 300: 130 tiles) and by the grouped tile (100 x 736:
+    299 tiles)."""
     import method_b200 as mb
     from oracle import port
-    cfg = config(nx, ny, 0, weno, bcs)
+    cfg = dict(config(nx, ny, 0, weno, bcs), model=model, sigma=5.0)
     sim = mb.Simulation(**cfg)
     p = sim.zeros(sim.Nprims)
     X, Y = np.meshgrid(np.linspace(0, 1, sim.Nx), np.linspace(0, 1, sim.Ny), indexing="ij")
     hot = ((X - 0.5) ** 2 + (Y - 0.4) ** 2 < 0.06)[:, :, None]
-    p[0] = np.where(hot, 1.0, 0.1)
-    p[4] = np.where(hot, 10.0, 0.05)
+    # SRRMHD's secant recovery does not take the strong blast
+    p[0] = np.where(hot, 1.0, 0.1 if model == "srmhd" else 0.8)
+    p[4] = np.where(hot, 10.0, 0.05) if model == "srmhd" else np.where(hot, 1.0, 0.7)
     p[1] = 0.3 * np.sin(7 * Y)[:, :, None]
     p[5], p[6] = 0.2, 0.1 * np.cos(5 * X)[:, :, None]
+    if model == "srrmhd":
+        p[9], p[10] = p[1] * p[7], -p[1] * p[6]
     sim.set_prims(p)
     o = port.PortSim(p, **cfg)
     dt = 0.05 / max(nx, ny)
