@@ -692,7 +692,8 @@ __device__ __forceinline__ bool imex_fast_form(const Grid& g, long long cell,
   }
   // D has no source: x[0] = c[0] throughout, so the conductivity is fixed per cell
   const double a = FORM <= 3 ? dt * kGam : 0.5 * dt, cp2 = g.cp * g.cp, sg = sigma_of(g, c[0]);
-  const double ip = rcp64(1 + a * rcp64(cp2));
+  // library divisions: cp is the caller's, and cp^2 may be infinite or subnormal
+  const double ip = 1 / (1 + a / cp2);
   x[12] = c[12] * ip;
   x[11] = (c[11] + a * c[13]) * ip;
   // the inner recovery's Z: the network's guess for the stage's first
