@@ -692,8 +692,10 @@ __device__ __forceinline__ bool imex_fast_form(const Grid& g, long long cell,
   }
   // D has no source: x[0] = c[0] throughout, so the conductivity is fixed per cell
   const double a = FORM <= 3 ? dt * kGam : 0.5 * dt, cp2 = g.cp * g.cp, sg = sigma_of(g, c[0]);
-  // library divisions: cp is the caller's, and cp^2 may be infinite or subnormal
-  const double ip = 1 / (1 + a / cp2);
+  // cp is the caller's: cp^2 may be infinite or subnormal, which rcp64 does not
+  // take; beyond 2^+-1000 its size changes nothing (two library divisions instead:
+  // SSP2 512x1024 step 0.2% slower)
+  const double ip = rcp64(1 + a * rcp64(fmin(fmax(cp2, 0x1p-1000), 0x1p1000)));
   x[12] = c[12] * ip;
   x[11] = (c[11] + a * c[13]) * ip;
   // the inner recovery's Z: the network's guess for the stage's first
