@@ -517,6 +517,65 @@ __global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
   tally_flush(tl, t < t_end, w.counters);
 }
 
+// The starting points of a batched recovery's cell: (v^2, rho h W^2) of the
+// previous primitive state in `prev`, of the chosen guess in `x`.
+__device__ __forceinline__ void batch_guesses(long long n, long long q, const srmhd::Residual& R,
+                                              int guess, const double* prims, const double* aux,
+                                              const double* __restrict__ zguess, double* prev,
+                                              double* x) {
+  double pg[4];
+#pragma unroll
+  for (int v = 0; v < 4; ++v) pg[v] = prims[v * n + q];
+  srmhd::guess_from_prims(pg, aux[q], prev);
+  if (guess == 1) {
+    x[0] = zguess[n + q];
+    x[1] = zguess[q];
+  } else if (guess == 2) {
+    const double E = R.tau + R.D;
+    x[1] = fmax(E, sqrt(R.Ssq) * 1.0000001);
+    x[0] = fmin(R.Ssq / (x[1] * x[1]), 0.999999);
+  } else {
+    x[0] = prev[0];
+    x[1] = prev[1];
+  }
+}
+
+// rcp64's reciprocals of Z^2 (Z + B^2)^2 need that product, which lies between
+// D^4 and about (8 (tau + D + B^2))^4, in the normal range.
+__device__ __forceinline__ bool newton_rcp_range(const srmhd::Residual& R) {
+  return R.D >= 0x1p-250 && fabs(R.tau) + R.D + R.Bsq <= 0x1p240;
+}
+
+struct BatchFallback {
+  double x0, x1;
+  int its, ok, fb;
+};
+
+// A cell that Newton's straight-line form left: Newton with the library's
+// division and rsqrt if its scale is out of that form's range, then the Powell
+// hybrid.  From memory, so that the caller keeps nothing for it.
+__device__ __noinline__ BatchFallback batch_fallback(long long n, long long q, double gamma,
+                                                     int guess, const double* cons,
+                                                     const double* prims, const double* aux,
+                                                     const double* zguess) {
+  double c[9], prev[2], x[2];
+#pragma unroll
+  for (int v = 0; v < 9; ++v) c[v] = cons[v * n + q];
+  const srmhd::Residual R = srmhd::residual_args(c, gamma);
+  batch_guesses(n, q, R, guess, prims, aux, zguess, prev, x);
+  int its = 0, fb = 0;
+  if (!newton_rcp_range(R)) {
+    for (int k = 0; k < (guess != 0 ? 2 : 1); ++k) {
+      if (newton_srmhd<false>(R.D, R.tau, R.BS * R.BS, R.Bsq, R.Ssq, gamma, x[1], x[0], its))
+        return {x[0], x[1], its, 1, fb};
+      fb = 1;
+      x[1] = prev[1];
+    }
+  }
+  const HybrdOut r = hybrd2_fallback(R, prev[0], prev[1]);
+  return {r.x0, r.x1, its + r.nfev, r.info == 1, 1};
+}
+
 // Batched SRMHD primitive recovery for independent cells: METHOD 0 the
 // reference's Powell hybrid, 1 Newton with the fallbacks of the grid
 // recovery.  Each method has its kernel, so that Newton's registers (80, 6
@@ -535,43 +594,27 @@ __global__ void __launch_bounds__(128, METHOD == 1 ? 6 : 5)
 #pragma unroll
     for (int v = 0; v < 9; ++v) c[v] = cons[v * n + q];
     srmhd::Residual R = srmhd::residual_args(c, gamma);
-    double prev[2];
-    {
-      double pg[4];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) pg[v] = prims[v * n + q];
-      srmhd::guess_from_prims(pg, aux[q], prev);
-    }
-    double x[2];
-    if (guess == 1) {
-      x[0] = zguess[n + q];
-      x[1] = zguess[q];
-    } else if (guess == 2) {
-      const double E = R.tau + R.D;
-      x[1] = fmax(E, sqrt(R.Ssq) * 1.0000001);
-      x[0] = fmin(R.Ssq / (x[1] * x[1]), 0.999999);
-    } else {
-      x[0] = prev[0];
-      x[1] = prev[1];
-    }
+    double prev[2], x[2];
+    batch_guesses(n, q, R, guess, prims, aux, zguess, prev, x);
     double p[8], a[13];
     int it = 0;
     bool ok = false;
     if constexpr (METHOD == 1) {
       const double BS2 = R.BS * R.BS;
+      const bool in_range = newton_rcp_range(R);
       ok = newton_srmhd<true>(R.D, R.tau, BS2, R.Bsq, R.Ssq, gamma, x[1], x[0], it);
       if (!ok && guess != 0) {
         fb = 1;
         x[1] = prev[1];
         ok = newton_srmhd<true>(R.D, R.tau, BS2, R.Bsq, R.Ssq, gamma, x[1], x[0], it);
       }
-      if (!ok) {
-        fb = 1;
-        const HybrdOut r = hybrd2_fallback(R, prev[0], prev[1]);
+      if (!ok || !in_range) {
+        const BatchFallback r = batch_fallback(n, q, gamma, guess, cons, prims, aux, zguess);
         x[0] = r.x0;
         x[1] = r.x1;
-        it += r.nfev;
-        ok = r.info == 1;
+        it = (in_range ? it : 0) + r.its;
+        ok = r.ok;
+        fb = r.fb;
       }
       from_solution_fast(c, x, gamma, R.BS, R.Bsq, R.Ssq, p, a);
     } else {

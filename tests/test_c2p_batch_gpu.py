@@ -48,3 +48,29 @@ def test_batch_recovers_generating_states(n, method, guess):
     assert np.max(np.abs(got[1:4] - p[1:4])) < 1e-8
     assert np.array_equal(got[5:8], p[5:8])
     assert np.max(np.abs(aux[0] - h) / h) < 1e-7  # h - 1 is down to 4e-3 of h
+
+
+@pytest.mark.parametrize("log4,guess", [(-123, 0), (-123, 2), (-100, 0), (100, 0), (122, 2)])
+def test_batch_recovers_states_of_any_scale(log4, guess):
+    """Newton on states scaled by powers of 4 (density, pressure and energy by s,
+    fields by sqrt(s): a symmetry of the equations, exact in binary) up to
+    where Z^2 (Z + B^2)^2 spans the range of doubles; same bound as above."""
+    import torch
+
+    from method_b200 import _lib
+    L = _lib.load()
+    n, s = 4096, 4.0 ** log4
+    p = initial.random_c2p_states(n, seed=1)
+    p[[0, 4]] *= s
+    p[5:8] *= 2.0 ** log4
+    cons, h = conserved(p)
+    pg, ag = np.zeros((8, n)), np.zeros((13, n))
+    pg[0], pg[1:4], ag[0] = p[0] * 1.01, p[1:4] * 0.99, h * 1.01
+    dc, dp, da = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (cons, pg, ag))
+    st = _lib.C2PBatchStats()
+    rc = L.mth_c2p_batch(G, n, dc.data_ptr(), dp.data_ptr(), da.data_ptr(), 1, guess, None, None,
+                         None, C.byref(st))
+    assert rc == 0 and st.cells == n and st.unconverged == 0
+    got = dp.cpu().numpy()
+    assert np.max(np.abs(got[0] - p[0]) / p[0]) < 1e-8
+    assert np.max(np.abs(got[1:4] - p[1:4])) < 1e-8
