@@ -173,7 +173,6 @@ __global__ void k_weno_dir(Grid g, int nc, int dir, const double* __restrict__ f
 // k_weno_dir for a runtime order.  Grids of fewer than two blocks per SM split
 // the variables over blocks, too: their threads wait for one reconstruction
 // after the other otherwise.
-int device_sm_count();
 template <bool ALL>
 void weno_dir_launch(const Grid& g, int nc, int order, int dir, const double* fplus,
                      const double* fminus, double* frecon, cudaStream_t st) {
@@ -654,13 +653,6 @@ template <class M>
 constexpr int kFp64SmallGroup = std::is_same<M, HYBRID>::value ? 5 : 3;
 template <int ORDER>
 constexpr int kFp64Blocks = ORDER <= 5 ? 4 : ORDER <= 7 ? 3 : 2;
-
-int device_sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  return sms;
-}
 
 template <class M, int ORDER, int TI, int G>
 cudaError_t fvs2d_group_ctas(const Grid& g, const double* cons, const double* prims,

@@ -579,11 +579,12 @@ __device__ __noinline__ BatchFallback batch_fallback(long long n, long long q, d
 // Batched SRMHD primitive recovery for independent cells: METHOD 0 the
 // reference's Powell hybrid, 1 Newton with the fallbacks of the grid
 // recovery.  Each method has its kernel, so that Newton's registers (80, 6
-// CTAs on an SM) and code are not the hybrid's (156 for both).  Bound by FP64
-// latency, then by memory (35 planes of 8 bytes): 2^22 cells from a
+// CTAs on an SM) and code are not the hybrid's (156 for both).  Newton is bound
+// by FP64 latency, then by memory (35 planes of 8 bytes): 2^22 cells from a
 // previous-step guess 0.47 -> 0.34 ms, 2.5 -> 3.5 TB/s.
-template <int METHOD>
-__global__ void __launch_bounds__(128, METHOD == 1 ? 6 : 5)
+// MINB: CTAs per SM the registers are sized for.
+template <int METHOD, int MINB>
+__global__ void __launch_bounds__(128, MINB)
     k_c2p_batch_srmhd(long long n, double gamma, int guess, const double* __restrict__ cons,
                       double* prims, double* aux, const double* __restrict__ zguess,
                       long long* counters) {
@@ -1117,10 +1118,16 @@ cudaError_t launch_c2p_batch(long long n, double gamma, int method, int guess,
                              const double* cons, double* prims, double* aux,
                              const double* zguess, long long* counters, cudaStream_t st) {
   const int b = (int)((n + 127) / 128);
+  // The hybrid's registers: 128 (4 CTAs) while its slowest cells decide, 96 (5
+  // CTAs, spills) once a launch has 16 CTAs per SM and more warps pay.  From a
+  // guess 1% off, 4 against 5 CTAs: 100 cells 236, 242 us; 10^4 693, 709; 8 10^4 1568,
+  // 1606; 3 10^5 2364, 2390; 10^6 6720, 6330; 2^22 23100, 21200.
   if (method == 1)
-    k_c2p_batch_srmhd<1><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
+    k_c2p_batch_srmhd<1, 6><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
+  else if (b < 16 * device_sm_count())
+    k_c2p_batch_srmhd<0, 4><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
   else
-    k_c2p_batch_srmhd<0><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
+    k_c2p_batch_srmhd<0, 5><<<b, 128, 0, st>>>(n, gamma, guess, cons, prims, aux, zguess, counters);
   return cudaGetLastError();
 }
 

@@ -24,6 +24,14 @@ enum ErrFlag : long long {
   ERR_DEVICE = 4,    // a bounded device-side wait ran out (tensor-core inference)
 };
 
+// SMs of the current device; 0 if it cannot be asked.
+inline int device_sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  return sms;
+}
+
 // Data::initData geometry (simData.cc:61-97) for a configuration; returns
 // false for a configuration the reference rejects.  `c` is an mth_config.
 bool grid_from_config(const void* c, Grid* g);

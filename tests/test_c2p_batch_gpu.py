@@ -74,3 +74,28 @@ def test_batch_recovers_states_of_any_scale(log4, guess):
     got = dp.cpu().numpy()
     assert np.max(np.abs(got[0] - p[0]) / p[0]) < 1e-8
     assert np.max(np.abs(got[1:4] - p[1:4])) < 1e-8
+
+
+def test_hybrid_register_variants_agree():
+    """The Powell hybrid's kernels on either side of their dispatch (16 CTAs of
+    128 cells per SM): the same cells give the same bits."""
+    import torch
+
+    from method_b200 import _lib
+    L = _lib.load()
+    line = 16 * 128 * torch.cuda.get_device_properties(0).multi_processor_count
+    p = initial.random_c2p_states(line, seed=2)
+    cons, h = conserved(p)
+    out = []
+    for n in (line - 128, line):
+        pg, ag = np.zeros((8, n)), np.zeros((13, n))
+        pg[:5], ag[0] = p[:5, :n], h[:n]
+        dc, dp, da = (torch.from_numpy(np.ascontiguousarray(x)).cuda()
+                      for x in (cons[:, :n], pg, ag))
+        st = _lib.C2PBatchStats()
+        rc = L.mth_c2p_batch(G, n, dc.data_ptr(), dp.data_ptr(), da.data_ptr(), 0, 0, None, None,
+                             None, C.byref(st))
+        assert rc == 0 and st.unconverged == 0
+        out.append((dp.cpu().numpy()[:, :line - 128], da.cpu().numpy()[:, :line - 128]))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
