@@ -54,9 +54,11 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
 
 static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
 
-// Quotients by one positive divisor, x / d, for many x of any size: RN(1 / d)
-// once (the bound above holds with h = 1/2), then three operations for an x
-// of 2^-900 to 2^900; zeros keep their sign, any other x divides as IEEE does.
+// Quotients by one divisor, x / d, for many x of any size, all rounded like
+// IEEE division.  d from 2^-100 to 2^100 (but the edge above): RN(1 / d) once (the
+// bound above holds with h = 1/2), then three operations for an x of 2^-900 to
+// 2^900, none for a zero.  Any other x or d (negative, zero, infinite, NaN)
+// divides, out of line.
 struct Divisor {
   double d, y;
   unsigned span;
@@ -67,7 +69,7 @@ struct Divisor {
   __device__ __forceinline__ double operator()(double x) const {
     const unsigned hi = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
     if (hi - (123u << 20) < span) return div_by(x, d, y);
-    return x == 0.0 ? x : div_ieee(x, d);
+    return x == 0.0 && span ? x : div_ieee(x, d);
   }
 };
 

@@ -79,3 +79,28 @@ def test_fused_step_matches_oracle(weno, nx, ny, model, bcs):
         assert np.array_equal(got, want), name
     sim.close()
     o.close()
+
+
+@pytest.mark.parametrize("bounds", [dict(xmin=1.0), dict(ymax=0.0), dict(xmin=2.0),
+                                    dict(xmax=float("nan")), dict(xmax=float("inf"))])
+@pytest.mark.parametrize("nx,ny", [(20, 24), (2368, 4)])
+def test_cell_size_of_any_kind_matches_oracle(bounds, nx, ny):
+    """Face fluxes, zeros among them, over cell sizes that are zero, negative,
+    NaN or infinite: what IEEE division gives (0 / 0 is NaN), by a CTA per
+    variable and by the grouped tile (296 tiles; few cells, as the retry of
+    failed recoveries is serial)."""
+    import method_b200 as mb
+    from oracle import port
+    cfg = dict(config(nx, ny, 0, 3, "outflow"), **bounds)
+    sim = mb.Simulation(**cfg)
+    p = sim.zeros(sim.Nprims)
+    p[0], p[4] = 1.0, 1.0
+    p[1, sim.Nx // 2:] = 0.1 * np.sin(np.arange(sim.Ny))[:, None]
+    p[5, sim.Nx // 2:] = 0.3
+    sim.set_prims(p)
+    o = port.PortSim(p, **cfg)
+    sim.step(1e-3)
+    o.step_dt(1e-3)
+    assert np.array_equal(sim.state()[0], o.state()[0], equal_nan=True)
+    sim.close()
+    o.close()
