@@ -49,7 +49,8 @@ __device__ __forceinline__ long long imex_cell(const Grid& g, long long cell,
 #pragma unroll
     for (int v = 0; v < 14; ++v) {
       f1[v] = flux1[v * N + cell];
-      s1[v] = source1[v * N + cell];
+      // the mixed stage 2 fills only the planes that have a source
+      s1[v] = SRRMHD::sourced(v) ? source1[v * N + cell] : 0.0;
       x[v] = 0.5 * (u[v] + u1[v * N + cell] - dt * f1[v]);
     }
   }

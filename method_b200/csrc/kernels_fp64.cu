@@ -566,7 +566,9 @@ __global__ void k_ssp2_combine(Grid g, int nc, double* cons, const double* __res
   const long long cell = cell_id(g, i, j, k);
   for (int v = 0; v < nc; ++v) {
     const long long o = v * g.Ntot + cell;
-    cons[o] += -0.5 * dt * (flux1[o] + flux2[o] - source1[o] - source2[o]);
+    // as in imex_cell, of stage 1's source only these planes count
+    const double s1 = SRRMHD::sourced(v) ? source1[o] : 0.0;
+    cons[o] += -0.5 * dt * (flux1[o] + flux2[o] - s1 - source2[o]);
   }
 }
 

@@ -27,3 +27,21 @@ def ref():
     if not R.available():
         pytest.skip("oracle/_ref not built (needs the reference sources)")
     return R
+
+
+@pytest.fixture(scope="session")
+def kernel_checks(tmp_path_factory):
+    """tests/cpp/kernel_checks.cu, built against the library's headers and linked to it."""
+    import ctypes
+    import subprocess
+
+    from method_b200 import _lib, build
+    _lib.load()
+    so = str(tmp_path_factory.mktemp("checks") / "kernel_checks.so")
+    src = os.path.join(ROOT, "tests", "cpp", "kernel_checks.cu")
+    r = subprocess.run([build.NVCC] + build.ARCH + build.COMMON +
+                       ["-fmad=false", "-shared", src, "-o", so, _lib.LIB_PATH,
+                        "-Xlinker", "-rpath," + os.path.dirname(_lib.LIB_PATH)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return ctypes.CDLL(so)
