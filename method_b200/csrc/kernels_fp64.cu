@@ -638,21 +638,35 @@ __global__ void __launch_bounds__(128)
 
 // The plain tile runs in passes of kFp64Group variables (fvs2d_group.cuh)
 // with registers sized for kFp64Blocks CTAs per SM: WENO3/5 4 CTAs (64
-// registers, a few spilled), WENO7 3, WENO9/11 2.  OT 1024^2 WENO5: two
-// passes of 5 + 4 variables 0.515 ms per launch, three of 3 0.549 ms (0.600
-// at 3 CTAs per SM), the one-pass tile 0.66 ms.
+// registers, a few spilled), WENO7 3, WENO9/11 2.  OT 1024^2 WENO5 RK2 step: two
+// passes of 5 + 4 variables 1.51 ms (1.53 at 3 CTAs per SM), three of 3 1.55, all
+// in one pass 1.67.
 // Grids of fewer than two tiles per SM run one CTA per tile and group of
 // variables: of one variable while that makes at most four CTAs per SM, else of
 // three (five for the Hybrid model, whose flux costs more to evaluate again
-// per group).  Plain RK2 steps with the tile's variables in one CTA, one per
-// CTA, three per CTA: KH 64 x 128 WENO3 (32 tiles) 65, 47, 50 us; OT 128 x 128
-// WENO5 (64) 87, 68, 71; 200 x 256 (200) 107, 98, 94; SRRMHD 200 x 256 96, 78, 63;
-// 256 x 288 (288) 86, 97, 86.  At two tiles per SM and above the grouped tile
-// is as fast with fewer loads.  All forms give the same bits.
+// per group; all of SRMHD's with WENO9/11 towards two tiles per SM).  Plain RK2
+// steps of Orszag-Tang grids one after another, us, with one variable per CTA,
+// three, five, all in one CTA, and in passes:
+//   SRMHD WENO5   64 x 128 (32 tiles) 59 63 69 82 91, 200 x 256 (200) 110 107 107 118 124,
+//                 256 x 288 (288) 134 122 124 122 127, 512 x 512 (1024) 403 349 359 345 347
+//   SRRMHD WENO5  128 x 128 (64) 57 50 54 77 92, 200 x 256 115 89 97 134 129,
+//                 256 x 288 153 119 118 141 133
+//   Hybrid WENO5  128 x 128 115 108 105 128 155, 200 x 256 193 167 163 193 197,
+//                 512 x 512 825 636 581 624 561
+//   SRMHD WENO7   128 x 128 97 93 103 137 145, 200 x 256 164 158 146 178 185
+//   SRMHD WENO9   240 x 256 (240) 270 218 244 242 249, 280 x 256 (280): three 250, all 245
+//   SRMHD WENO11  232 x 256 (232): three 291, all 315; 264 x 256 (264) 340, 320
+//   SRRMHD WENO11 128 x 128 199 167 155 263 311, 256 x 288 592 468 458 521 465
+// All forms give the same bits.
 template <class M>
 constexpr int kFp64Group = 5;
 template <class M>
 constexpr int kFp64SmallGroup = std::is_same<M, HYBRID>::value ? 5 : 3;
+// Tiles per SM above which (and below two) SRMHD's WENO9/11, whose wide halo each
+// group loads and splits again, run one CTA per tile with all variables.
+template <class M, int ORDER>
+constexpr double kFp64WholeTile =
+    !std::is_same<M, SRMHD>::value ? 0.0 : ORDER == 9 ? 1.75 : ORDER == 11 ? 1.67 : 0.0;
 template <int ORDER>
 constexpr int kFp64Blocks = ORDER <= 5 ? 4 : ORDER <= 7 ? 3 : 2;
 
@@ -688,6 +702,11 @@ cudaError_t fvs2d_instance(const Grid& g, const double* cons, const double* prim
   }
   if (tiles * M::NC <= 4LL * sms)
     return fvs2d_group_ctas<M, ORDER, TI, 1>(g, cons, prims, aux, u0, out, dt, mode, tail, grid, st);
+  if constexpr (kFp64WholeTile<M, ORDER> > 0) {
+    if (tiles > kFp64WholeTile<M, ORDER> * sms)
+      return fvs2d_group_ctas<M, ORDER, TI, M::NC>(g, cons, prims, aux, u0, out, dt, mode, tail,
+                                                   grid, st);
+  }
   return fvs2d_group_ctas<M, ORDER, TI, kFp64SmallGroup<M>>(g, cons, prims, aux, u0, out, dt, mode,
                                                             tail, grid, st);
 }
