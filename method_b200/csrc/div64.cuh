@@ -11,7 +11,8 @@
 // correction (P. Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).
 //   y = y0 (1 + e + e^2 + e^3), e = 1 - b y0, from the hardware's
-//   approximation y0 (|e| <= 2^-18): |y - 1/b| <= (1/2 + 2^-18) ulp;
+//   approximation y0 (of b's high word: |e| <= 2^-18, tested over all significands
+//   of 20 bits, tests/test_div64_gpu.py): |y - 1/b| <= (1/2 + 2^-18) ulp;
 //   q0 = RN(a y), r = a - b q0, q = RN(q0 + r y).
 // Why q = RN(a / b) when b's significand B is at most 2 - 2^-15 and neither
 // a y nor r leaves the normal range.  Let A be a's significand, h = 1/2 + 2^-18.
@@ -72,5 +73,21 @@ struct Divisor {
     return x == 0.0 && span ? x : div_ieee(x, d);
   }
 };
+
+// 1/x and 1/sqrt(x) for the mixed form, without the branches of the library's
+// division and rsqrt, by Newton's series from the hardware's approximations:
+// of a normal x (rsqrt64: a positive one) whose reciprocal is normal too, to
+// 0.51 and 1.2 ulp (x y0^2 = 1 - e, |e| < 2^-18, for the root y = y0 (1 + e/2 + 3/8 e^2
+// + ...), whose e^3 term is below 2^-55).  An infinite, zero or subnormal x gives
+// NaN, a reciprocal below 2^-1022 gives 0: callers keep their operands away from
+// there.  The recoveries are chains of them at 40-48% of the FP64 pipe, bound by
+// the chains' latency.
+__device__ __forceinline__ double rcp64(double x) { return div_rcp(x); }
+__device__ __forceinline__ double rsqrt64(double x) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+  const double e = fma(-(x * y0), y0, 1.0);
+  return fma(y0 * e, fma(0.375, e, 0.5), y0);
+}
 
 }  // namespace mth

@@ -31,20 +31,6 @@ namespace mth {
 
 namespace {
 
-// 1/x and 1/sqrt(x) of a normal positive (rcp: or negative) x to about one ulp,
-// without the branches of the library's division and rsqrt: Newton's series
-// from the hardware's approximations, x y0^2 = 1 - e with |e| < 2^-18 (for the
-// root y = y0 (1 + e/2 + 3/8 e^2 + ...); the e^3 term is below 2^-55).  The
-// recoveries are chains of them at 40-48% of the FP64 pipe, bound by the
-// chains' latency.
-__device__ __forceinline__ double rcp64(double x) { return div_rcp(x); }
-__device__ __forceinline__ double rsqrt64(double x) {
-  double y0;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
-  const double e = fma(-(x * y0), y0, 1.0);
-  return fma(y0 * e, fma(0.375, e, 0.5), y0);
-}
-
 // Newton in Z for SRMHD, safeguarded by a bracket.  v^2(Z) above is strictly
 // decreasing for Z > 0, so "v^2 >= 1 or g < 0" marks the left of the root
 // and g > 0 its right; a Newton step that leaves the bracket (or a zero or

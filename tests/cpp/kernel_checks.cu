@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "launch.h"
+#include "weno.cuh"
 
 namespace {
 
@@ -79,4 +80,66 @@ extern "C" int run_ssp2_combine(const void* cfg, double* cons, const double* flu
   if (b.e == cudaSuccess) b.e = cudaDeviceSynchronize();
   b.down(cons, c, n);
   return b.e;
+}
+
+namespace {
+
+// out[k n + i]: 0 div_by (y = div_rcp(b)), 1 Divisor(b)(a), 2 IEEE a / b, 3 rcp64(b),
+// 4 rsqrt64(b), 5 and 6 the residuals 1 - b y0 and 1 - b y0^2 of the hardware's
+// approximations of 1/b and 1/sqrt(b).
+__global__ void k_quotients(int n, const double* a, const double* b, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double x = a[i], d = b[i];
+  out[i] = mth::div_by(x, d, mth::div_rcp(d));
+  out[n + i] = mth::Divisor(d)(x);
+  out[2 * n + i] = x / d;
+  out[3 * n + i] = mth::rcp64(d);
+  out[4 * n + i] = mth::rsqrt64(d);
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  out[5 * n + i] = __fma_rn(-d, y, 1.0);
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  out[6 * n + i] = __fma_rn(-(d * y), y, 1.0);
+}
+
+// out[k n + i]: the face of stencils v[2 ORDER * i ...] (ORDER cells upwind, ORDER
+// downwind, in the order the points take them) by weno_face_exact with one
+// operand test (0) and with two (1), and with IEEE divisions (2).
+template <int ORDER>
+__global__ void k_faces(int n, const double* v, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double* p = v + 2 * ORDER * i;
+  const double* m = p + 2 * ORDER - 1;  // read downwards
+  out[i] = mth::weno_face_exact<ORDER, true>(p, m, 1);
+  out[n + i] = mth::weno_face_exact<ORDER, false>(p, m, 1);
+  out[2 * n + i] = mth::weno_face_ieee<ORDER>(p, m, 1);
+}
+
+}  // namespace
+
+extern "C" int run_quotients(int n, const double* a, const double* b, double* out) {
+  Buffers m;
+  const double *x = m.up(a, n), *d = m.up(b, n);
+  double* o = m.up<double>(nullptr, 7LL * n);
+  if (m.e != cudaSuccess) return m.e;
+  k_quotients<<<(n + 127) / 128, 128>>>(n, x, d, o);
+  m.e = cudaDeviceSynchronize();
+  m.down(out, o, 7LL * n);
+  return m.e;
+}
+
+extern "C" int run_faces(int order, int n, const double* v, double* out) {
+  Buffers m;
+  const double* x = m.up(v, 2LL * order * n);
+  double* o = m.up<double>(nullptr, 3LL * n);
+  if (m.e != cudaSuccess) return m.e;
+  if (order == 3)
+    k_faces<3><<<(n + 127) / 128, 128>>>(n, x, o);
+  else
+    k_faces<5><<<(n + 127) / 128, 128>>>(n, x, o);
+  m.e = cudaDeviceSynchronize();
+  m.down(out, o, 3LL * n);
+  return m.e;
 }
