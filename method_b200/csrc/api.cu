@@ -183,10 +183,11 @@ cudaError_t flux_stage(mth_handle* h, double* c, double* p, double* a, const dou
                        double* out, double dt, int mode) {
   const bool srmhd = h->cfg.model == MTH_SRMHD;
   const double in = srmhd ? 22 : 24, nc = h->NC;
-  // flux inputs + the written state (+ u0 for the corrector; + u0, flux1,
-  // source1 and the 6 source inputs for the fused SSP2 closing stage)
+  // flux inputs + the written state (+ u0 for the corrector; + u0, flux1 and
+  // SRRMHD's 5 sourced planes of source1 for the fused SSP2 closing stage, whose
+  // own source reads flux inputs)
   const double dpc = in + nc + (mode == STAGE_RK2_CORR ? nc : 0) +
-                     (mode == STAGE_SSP2_FINAL ? 3 * nc + 6 : 0);
+                     (mode == STAGE_SSP2_FINAL ? 2 * nc + 5 : 0);
   const char* name = h->fused ? (h->cfg.precision == MTH_MIXED ? "fvs2d_fp32" : "fvs2d_fp64")
                               : "fvs_generic";
   return timed(h, name, dpc, [&] { return flux_stage_raw(h, c, p, a, u0, out, dt, mode); });
@@ -285,7 +286,7 @@ cudaError_t rksplit2_half_source(mth_handle* h, double dt) {
     // reads any, and of prims alone
     const RegimeWork* w = h->cfg.regime ? &h->regime : nullptr;
     if (w && (e = launch_apply_bcs(h->g, h->prims, h->NP, h->st))) return e;
-    if ((e = timed(h, "source", 2.0 * h->NC, [&] {
+    if ((e = timed(h, "source", 2.0 * h->NC + 3, [&] {
            return launch_hybrid_source_add(h->g, h->cfg.weno_order, h->cons, h->prims, h->aux, w,
                                            h->hext, h->cfg.precision == MTH_MIXED, 0.5 * dt,
                                            h->st);
@@ -397,7 +398,7 @@ cudaError_t enqueue_ssp2_part(mth_handle* h, double dt, int part) {
          })))
       return e;
     if ((e = flux_stage(h, h->u2, h->prims, h->aux, nullptr, h->flux2, dt, STAGE_FNET))) return e;
-    if ((e = timed(h, "ssp2_combine", 6.0 * h->NC, [&] {
+    if ((e = timed(h, "ssp2_combine", 5.0 * h->NC + 5, [&] {
            return launch_ssp2_combine(h->g, h->NC, h->cons, h->flux1, h->flux2, h->src1, h->src2,
                                       dt, h->st);
          })))
@@ -410,7 +411,11 @@ cudaError_t enqueue_ssp2_part(mth_handle* h, double dt, int part) {
        })))
     return e;
   if ((e = flux_stage(h, h->u1, h->prims, h->aux, nullptr, h->flux1, dt, STAGE_FNET))) return e;
-  if ((e = timed(h, fast ? "imex_newton_stage2" : "imex_hybrd_stage2", fast ? 54 : 71, [&] {
+  // cons, flux1, aux[10] in and the stage out, with the 5 sourced planes of
+  // source1: in and u1 too (exact solve); out, from 3 planes of u1 and 3 of aux;
+  // or in, with the network's Z (its own passes come on top)
+  const double dpc = !fast ? 62 : mlp_work(h) ? 49 : 54;
+  if ((e = timed(h, fast ? "imex_newton_stage2" : "imex_hybrd_stage2", dpc, [&] {
          return fast ? launch_imex_fast(h->g, 2, h->cons, h->aux, h->u1, h->flux1, h->src1,
                                         h->u2, dt, imex_work(h), h->st, mlp_work(h))
                      : launch_imex_stage(h->g, 2, h->cons, h->aux, h->u1, h->flux1, h->src1,
