@@ -633,7 +633,9 @@ mth_status mth_create(const mth_config* cfg, mth_handle** out) {
   if ((e = alloc0(&h->prims, bytes(h, h->NP), h->st))) return bail("prims", e);
   if ((e = alloc0(&h->aux, bytes(h, h->NA), h->st))) return bail("aux", e);
   if (c.integrator == MTH_RK2 || c.integrator == MTH_RKSPLIT || c.integrator == MTH_RKSPLIT2) {
-    if (c.integrator == MTH_RKSPLIT2 && (e = alloc0(&h->hsrc, bytes(h, h->NC), h->st)))
+    // the half source steps of separate passes (rksplit2_half_source)
+    if (c.integrator == MTH_RKSPLIT2 && (c.model != MTH_HYBRID || g.functional_sigma) &&
+        (e = alloc0(&h->hsrc, bytes(h, h->NC), h->st)))
       return bail("source", e);
     if ((e = alloc0(&h->p1cons, bytes(h, h->NC), h->st))) return bail("p1cons", e);
     if ((e = alloc0(&h->p1prims, bytes(h, h->NP), h->st))) return bail("p1prims", e);

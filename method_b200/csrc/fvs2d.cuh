@@ -103,12 +103,10 @@ struct Fvs2dSmem {
 // CTAs per SM the FP32 tile's register allocation is sized for: enough for
 // 1024 resident threads (32 warps, 64 registers each) where shared memory
 // admits them (OT 1024^2 WENO5, TI 8: 0.220 -> 0.179 ms per launch against
-// the compiler's own 80-register choice).  The FP64 tile keeps the compiler's
-// choice (its shared memory admits two CTAs).
-template <class M, typename R, int ORDER, int TI>
+// the compiler's own 80-register choice).
+template <class M, int ORDER, int TI>
 constexpr int fvs2d_min_blocks() {
-  if (sizeof(R) == 8) return 1;
-  const int by_smem = (int)(220 * 1024 / Fvs2dSmem<M, R, ORDER, TI>::bytes);
+  const int by_smem = (int)(220 * 1024 / Fvs2dSmem<M, float, ORDER, TI>::bytes);
   const int by_threads = 1024 / (32 * TI);
   const int b = by_smem < by_threads ? by_smem : by_threads;
   return b < 1 ? 1 : b;
@@ -499,27 +497,28 @@ __device__ __forceinline__ void fvs2d_tile_pairs(const Grid& g, const double* __
   stage_update<M, float>(g, cons, aux, u0, out, dt, mode, tail, cell_id(g, ci, cj, 0), acc);
 }
 
-// The stage's tile in the form that serves R and ORDER.
-template <class M, typename R, int ORDER, int TI>
-__device__ __forceinline__ void fvs2d_any_tile(const Grid& g, const double* __restrict__ cons,
-                                               const double* __restrict__ prims,
-                                               const double* __restrict__ aux, const double* u0,
-                                               double* out, double dt, int mode, int ti, int tj,
-                                               unsigned char* smem_raw, StageTail tail) {
-  if constexpr (sizeof(R) == 4 && ORDER <= 5)
+// The mixed form's tile of order ORDER.
+template <class M, int ORDER, int TI>
+__device__ __forceinline__ void fvs2d_fp32_tile(const Grid& g, const double* __restrict__ cons,
+                                                const double* __restrict__ prims,
+                                                const double* __restrict__ aux, const double* u0,
+                                                double* out, double dt, int mode, int ti, int tj,
+                                                unsigned char* smem_raw, StageTail tail) {
+  if constexpr (ORDER <= 5)
     fvs2d_tile_pairs<M, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti, tj, smem_raw, tail);
   else
-    fvs2d_tile<M, R, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti, tj, smem_raw, tail);
+    fvs2d_tile<M, float, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti, tj, smem_raw,
+                                    tail);
 }
 
-template <class M, typename R, int ORDER, int TI>
-__global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, R, ORDER, TI>()))
-    k_fvs2d(Grid g, const double* __restrict__ cons, const double* __restrict__ prims,
-            const double* __restrict__ aux, const double* u0, double* out, double dt,
-            int mode, StageTail tail, int ti0) {
+template <class M, int ORDER, int TI>
+__global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, ORDER, TI>()))
+    k_fvs2d_fp32(Grid g, const double* __restrict__ cons, const double* __restrict__ prims,
+                 const double* __restrict__ aux, const double* u0, double* out, double dt,
+                 int mode, StageTail tail, int ti0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  fvs2d_any_tile<M, R, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti0 + blockIdx.y,
-                                  blockIdx.x, smem_raw, tail);
+  fvs2d_fp32_tile<M, ORDER, TI>(g, cons, prims, aux, u0, out, dt, mode, ti0 + blockIdx.y,
+                                blockIdx.x, smem_raw, tail);
 }
 
 }  // namespace mth

@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(128, kSrrmhdMinBlocks)
 // ---------------------------------------------------------------------------
 // Ensemble kernels (mixed form).
 template <class M, int ORDER, int TI>
-__global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, float, ORDER, TI>()))
+__global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, ORDER, TI>()))
     k_ens_fvs_fp32(const Member* __restrict__ mem, const Item* __restrict__ items, int n_items,
                    int ic, int ip, int ia, int iu0, int iout, int mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -876,9 +876,9 @@ __global__ void __launch_bounds__(32 * TI, (fvs2d_min_blocks<M, float, ORDER, TI
     const Item w = items[it];
     const Member& d = mem[w.m];
     const Grid g = d.g;
-    fvs2d_any_tile<M, float, ORDER, TI>(g, d.a[ic], d.a[ip], d.a[ia],
-                                        iu0 >= 0 ? d.a[iu0] : nullptr, d.a[iout], d.dt, mode, w.a,
-                                        w.b, smem_raw, StageTail{d.a[EA_F1], d.a[EA_S1], g.cp});
+    fvs2d_fp32_tile<M, ORDER, TI>(g, d.a[ic], d.a[ip], d.a[ia], iu0 >= 0 ? d.a[iu0] : nullptr,
+                                  d.a[iout], d.dt, mode, w.a, w.b, smem_raw,
+                                  StageTail{d.a[EA_F1], d.a[EA_S1], g.cp});
     __syncthreads();
   }
 }
@@ -995,7 +995,7 @@ cudaError_t fvs2d_fp32_instance(const Grid& g, const double* cons, const double*
                                 const double* aux, const double* u0, double* out, double dt,
                                 int mode, StageTail tail, cudaStream_t st, int ti0, int nti) {
   using S = Fvs2dSmem<M, float, ORDER, TI>;
-  auto kern = k_fvs2d<M, float, ORDER, TI>;
+  auto kern = k_fvs2d_fp32<M, ORDER, TI>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
   if (e != cudaSuccess) return e;
