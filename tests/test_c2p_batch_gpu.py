@@ -99,3 +99,31 @@ def test_hybrid_register_variants_agree():
         out.append((dp.cpu().numpy()[:, :line - 128], da.cpu().numpy()[:, :line - 128]))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 128, 129, 1000])
+@pytest.mark.parametrize("method,guess", [(0, 0), (1, 0), (1, 2)])
+@pytest.mark.parametrize("bad", [False, True])
+def test_batch_statistics(n, method, guess, bad):
+    """n copies of one cell count n times what one counts: cells, iterations and,
+    for a cell that does not converge, failures and fallbacks."""
+    import torch
+
+    from method_b200 import _lib
+    L = _lib.load()
+    p = initial.random_c2p_states(1, seed=5)
+    cons, h = conserved(p)
+    if bad:
+        cons[1] = 100 * (cons[0] + cons[4])  # |S| far beyond tau + D
+    pg, ag = np.zeros((8, 1)), np.zeros((13, 1))
+    pg[:5], ag[0] = p[:5] * (0.99 if method else 1.0), h
+    counts = []
+    for m in (1, n):
+        dc, dp, da = (torch.from_numpy(np.repeat(x, m, axis=1)).cuda() for x in (cons, pg, ag))
+        st = _lib.C2PBatchStats()
+        rc = L.mth_c2p_batch(G, m, dc.data_ptr(), dp.data_ptr(), da.data_ptr(), method, guess, None,
+                             None, None, C.byref(st))
+        assert rc == (1 if bad else 0)
+        counts.append(np.array([st.cells, st.iterations, st.unconverged, st.fallbacks]))
+    assert counts[0][0] == 1 and counts[0][1] > 0 and counts[0][2] == bad
+    assert np.array_equal(counts[1], n * counts[0])
