@@ -753,7 +753,7 @@ def ncu_record(kernel):
 
 def fp64_pipe_roofline(inst_per_cell, cells, launch_ms, clk):
     """The FP64 pipe's roofline of a kernel whose FP64 work bounds it: thread
-    instructions (DADD + DMUL + DFMA, counted by ncu per interior cell) per
+    instructions (ncu's op_fp64_pred_on per interior cell) per
     launch over the CUDA-event launch time, against 64 FP64 thread
     instructions per SM per clock (ncu's peak_sustained of
     sm__sass_thread_inst_executed_op_dfma_pred_on on B200) x SMs x the median

@@ -1,17 +1,17 @@
 // Fused 2D flux stage, plain FP64 form, conserved variables in groups.
 //
-// The FP64 tile of fvs2d.cuh keeps f+ and f- of all NC variables of its
-// tile-plus-halo region in shared memory (85 KB for SRMHD WENO5 at 8 x 32),
-// which with its register count holds two CTAs, 16 warps, on an SM; its
-// WENO chains (IEEE divisions, no FMA contraction, the reference's order)
-// then wait on FP64 latency with too few warps to cover it.  This form runs
-// the same tile as G-variable passes: each pass loads the region's flux
-// inputs, evaluates the flux of only its G variables (the compiler drops
-// the rest, loads included, as they are plain loads), splits, reconstructs
-// and accumulates their x and then y differences in registers.  Shared memory
-// shrinks by NC / G and the register cap admits more CTAs per SM.  Every
-// value is computed by the same expression as in the one-pass tile, so the
-// result is bit-identical to it and to the reference.
+// With f+ and f- of all NC variables of its tile-plus-halo region in shared
+// memory (85 KB for SRMHD WENO5 at 8 x 32) and the registers of all their
+// differences, an SM holds two CTAs of the FP64 tile, 16 warps, and its WENO
+// chains (no FMA contraction, the reference's order) wait on FP64 latency
+// with too few warps to cover it.  This form runs the tile as G-variable
+// passes: each pass loads the region's flux inputs, evaluates the flux of only
+// its G variables (the compiler drops the rest, loads included, as they are
+// plain loads), splits, reconstructs and accumulates their x and then y
+// differences in registers.  Shared memory shrinks by NC / G and the register
+// cap admits more CTAs per SM.  On small grids the groups are CTAs of their own
+// (k_fvs2d_group_ctas).  Every value is computed by the same expression as in
+// fvs2d.cuh's tile, so the result is bit-identical to it and to the reference.
 #pragma once
 #include "fvs2d.cuh"
 

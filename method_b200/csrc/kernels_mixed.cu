@@ -567,7 +567,7 @@ __device__ __noinline__ BatchFallback batch_fallback(long long n, long long q, d
 // recovery.  Each method has its kernel, so that Newton's registers (80, 6
 // CTAs on an SM) and code are not the hybrid's (156 for both).  Newton is bound
 // by FP64 latency, then by memory (35 planes of 8 bytes): 2^22 cells from a
-// previous-step guess 0.47 -> 0.34 ms, 2.5 -> 3.5 TB/s.
+// previous-step guess 0.46 -> 0.31 ms, 2.6 -> 3.8 TB/s.
 // MINB: CTAs per SM the registers are sized for.
 template <int METHOD, int MINB>
 __global__ void __launch_bounds__(128, MINB)
