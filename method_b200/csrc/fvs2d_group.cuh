@@ -174,8 +174,9 @@ __device__ __forceinline__ void group_cta(const Grid& g, const double* __restric
   }
 }
 
-template <class M, int ORDER, int TI, int G>
-__global__ void __launch_bounds__(32 * TI)
+// MINB: CTAs per SM the registers are sized for, 0 for the compiler's choice.
+template <class M, int ORDER, int TI, int G, int MINB>
+__global__ void __launch_bounds__(32 * TI, MINB)
     k_fvs2d_group_ctas(Grid g, const double* __restrict__ cons, const double* __restrict__ prims,
                        const double* __restrict__ aux, const double* u0, double* out, double dt,
                        int mode, StageTail tail) {

@@ -667,6 +667,11 @@ constexpr int kFp64SmallGroup = std::is_same<M, HYBRID>::value ? 5 : 3;
 template <class M, int ORDER>
 constexpr double kFp64WholeTile =
     !std::is_same<M, SRMHD>::value ? 0.0 : ORDER == 9 ? 1.75 : ORDER == 11 ? 1.67 : 0.0;
+// SRRMHD's WENO7 in groups of three fits 64 registers, 4 CTAs per SM (32 bytes
+// spilled): the compiler's choice of 70, 3 CTAs, makes a 200 x 256 step 161 us, not 149.
+template <class M, int ORDER, int G>
+constexpr int kFp64CtasBlocks =
+    std::is_same<M, SRRMHD>::value && G == 3 && ORDER == 7 ? 4 : 0;
 template <int ORDER>
 constexpr int kFp64Blocks = ORDER <= 5 ? 4 : ORDER <= 7 ? 3 : 2;
 
@@ -675,7 +680,7 @@ cudaError_t fvs2d_group_ctas(const Grid& g, const double* cons, const double* pr
                              const double* aux, const double* u0, double* out, double dt, int mode,
                              StageTail tail, dim3 grid, cudaStream_t st) {
   using S = Fvs2dGroupSmem<M, ORDER, TI, G>;
-  auto kern = k_fvs2d_group_ctas<M, ORDER, TI, G>;
+  auto kern = k_fvs2d_group_ctas<M, ORDER, TI, G, kFp64CtasBlocks<M, ORDER, G>>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
   if (e != cudaSuccess) return e;
