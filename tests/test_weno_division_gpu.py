@@ -81,17 +81,24 @@ def test_fused_step_matches_oracle(weno, nx, ny, model, bcs):
     o.close()
 
 
-@pytest.mark.parametrize("bounds", [dict(xmin=1.0), dict(ymax=0.0), dict(xmin=2.0),
-                                    dict(xmax=float("nan")), dict(xmax=float("inf"))])
+BAND = 2.0 - 2.0 ** -16  # a significand that no branch-free quotient takes
+
+
+@pytest.mark.parametrize("dx,dy", [(0.0, 0.1), (0.1, 0.0), (-0.1, 0.1), (float("nan"), 0.1),
+                                   (float("inf"), 0.1), (BAND, 2.0), (0.125, BAND / 16),
+                                   (2.0 ** -99, 2.0 ** -99), (2.0 ** -101, 2.0 ** -101),
+                                   (2.0 ** 101, 2.0 ** 101)])
 @pytest.mark.parametrize("nx,ny", [(20, 24), (2368, 4)])
-def test_cell_size_of_any_kind_matches_oracle(bounds, nx, ny):
+def test_cell_size_of_any_kind_matches_oracle(dx, dy, nx, ny):
     """Face fluxes, zeros among them, over cell sizes that are zero, negative,
-    NaN or infinite: what IEEE division gives (0 / 0 is NaN), by a CTA per
-    variable and by the grouped tile (296 tiles; few cells, as the retry of
-    failed recoveries is serial)."""
+    NaN or infinite (0 / 0 is NaN), and on either side of the branch-free
+    quotients' limits: what IEEE division gives, by a CTA per variable and by
+    the grouped tile (296 tiles; few cells, as the retry of failed recoveries is
+    serial)."""
     import method_b200 as mb
     from oracle import port
-    cfg = dict(config(nx, ny, 0, 3, "outflow"), **bounds)
+    cfg = dict(config(nx, ny, 0, 3, "outflow"), xmax=dx * nx, ymax=dy * ny)
+    dt = 1e-2 * min(d for d in (dx, dy) if d > 0)
     sim = mb.Simulation(**cfg)
     p = sim.zeros(sim.Nprims)
     p[0], p[4] = 1.0, 1.0
@@ -99,8 +106,8 @@ def test_cell_size_of_any_kind_matches_oracle(bounds, nx, ny):
     p[5, sim.Nx // 2:] = 0.3
     sim.set_prims(p)
     o = port.PortSim(p, **cfg)
-    sim.step(1e-3)
-    o.step_dt(1e-3)
+    sim.step(dt)
+    o.step_dt(dt)
     assert np.array_equal(sim.state()[0], o.state()[0], equal_nan=True)
     sim.close()
     o.close()
